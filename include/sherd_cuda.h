@@ -301,15 +301,15 @@ int sherd_icp_rung(sherd_ctx *ctx, const double *source, uint32_t n_source,
  * is launched. The poses are read on the device only, so a non-finite one is
  * not refused up front: its rung finds no correspondence and the call returns
  * SHERD_E_INVALID after it ran; pass finite poses.
- * The per-point working memory (each source point's last match) lives in one
- * array inside this library, sized at SHERD_NOALLOC_CAPACITY entries and held
- * by every GPU that loads the library until the process exits; a call with
+ * The working memory (each source point's last match and how far it stands)
+ * lives in arrays inside this library, sized at SHERD_NOALLOC_CAPACITY points and
+ * held by every GPU that loads the library until the process exits; a call with
  * k * n_source above it is refused with SHERD_E_INVALID. The call allocates
- * nothing, waits for its own work, and leaves the array holding the last
- * call's contents (each rung resets the part it uses before reading it). All
- * calls share the one array, so two calls that overlap on the GPU (from two
+ * nothing, waits for its own work, and leaves the arrays holding the last
+ * call's contents (each rung writes the part it uses before reading it). All
+ * calls share them, so two calls that overlap on the GPU (from two
  * contexts, or two host threads on different contexts of one device) race.
- * The first call on each device looks the array's device address up
+ * The first call on each device looks the arrays' device addresses up
  * (cudaGetSymbolAddress) with that device current; make that first call
  * before any stream capture on the device. */
 #define SHERD_NOALLOC_CAPACITY (1u << 20)

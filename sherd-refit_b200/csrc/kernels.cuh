@@ -267,25 +267,29 @@ __global__ void k_cone_votes(MeshView m, const double *centroids, const double *
 
 // ---- ICP -----------------------------------------------------------------------
 
-// Executor::icp_rung: one block per candidate.
-__global__ void __launch_bounds__(ICP_BLOCK, 4) k_icp_rung(const double4 *src, uint32_t ns,
-                                                        CloudView tgt, const double *inits,
-                                                        sherd_icp_options opt, int *hints,
-                                                        sherd_registration *out, uint32_t *status) {
-  __shared__ IcpShared sh;
+// Executor::icp_rung: one block of 128 G threads, or one cluster of C of them,
+// per candidate.
+template <int G, int C>
+__global__ void __launch_bounds__(ICP_BLOCK *G, 4 / G)
+    k_icp_rung(const double4 *src, uint32_t ns, CloudView tgt, const double *inits,
+               sherd_icp_options opt, IcpMemory<int> mem, sherd_registration *out,
+               uint32_t *status) {
+  IcpBlock<G, C> &b = rung_memory<G, C>();
   uint32_t st = 0;
+  const uint32_t cand = blockIdx.x / C;
   if (threadIdx.x < 16) {
-    double v = inits[16 * blockIdx.x + threadIdx.x];
-    sh.t[threadIdx.x] = v;
+    double v = inits[16 * size_t(cand) + threadIdx.x];
+    b.s.t[threadIdx.x] = v;
     // A non-finite start (which only a caller passing device-resident poses can hand over,
     // the host-buffer entry refusing it first) is reported; the rung itself stays in bounds
     // (no distance compares below a NaN radius, so it finds no correspondence).
     if (!isfinite(v)) st |= ST_RANGE;
   }
   __syncthreads();
-  icp_rung_block(src, ns, tgt, opt.max_correspondence_distance, opt.max_iteration, sh,
-                 hints + size_t(ns) * blockIdx.x, out + blockIdx.x, st,
-                 opt.estimation == SHERD_POINT_TO_POINT);
+  icp_rung_block<G, C>(src, ns, tgt, opt.max_correspondence_distance, opt.max_iteration, b,
+                       memory_slot(mem, cand, ns), out + cand, st,
+                       opt.estimation == SHERD_POINT_TO_POINT);
+  rung_sync<C>();  // no CTA of a cluster ends while another may write to it
   if (st) atomicOr(status, st);
 }
 
@@ -349,15 +353,15 @@ __global__ void k_penetration_share(MeshView m, const double *pts, uint32_t n, P
 
 // ---- the batched stage-2 path ----------------------------------------------------
 
-// Resident ladder CTAs per SM a k_ladder variant's register budget is cut for
-// (65536 / (ICP_BLOCK * MINB) registers a thread at most). The batch picks a
-// variant per point-count bucket (the autotuner in sherd.cu); the last is the
-// default.
+// The forms k_ladder is built in. The first three are a block of 256 threads per
+// item with a register budget for so many resident CTAs per SM; the batch picks
+// one per point-count bucket (the autotuner in sherd.cu). The others are blocks
+// of 512 threads, alone or in clusters of 2, 4 and 8 per item, for batches with
+// fewer items than such blocks fill the device (ladder_form in sherd.cu).
 constexpr int LADDER_VARIANTS = 3;
-constexpr int LADDER_MINB[LADDER_VARIANTS] = {6, 8, 10};
+constexpr int LADDER_MINB[LADDER_VARIANTS] = {3, 4, 5};
 // The variant a bucket runs until the autotuner has timed it (and when it has
-// too few items to time): 8 CTAs per SM, which the 4-wide nearest-point walk
-// made 15-20 % faster than 10 on the collection.
+// too few items to time).
 constexpr int LADDER_DEFAULT = 1;
 
 struct QueueCtl {
@@ -391,45 +395,63 @@ __device__ __forceinline__ bool take(const QueueCtl &q, unsigned long long start
   return slot != 0xFFFFFFFFu;
 }
 
+// take() for a cluster of C blocks: the first block's answer for all of them.
+template <int C>
+__device__ __forceinline__ bool take_shared(const QueueCtl &q, unsigned long long start,
+                                            unsigned &slot, uint32_t &st) {
+  if constexpr (C == 1) {
+    return take(q, start, slot, st);
+  } else {
+    __shared__ unsigned s_got;
+    if (cta_rank<C>() == 0) {
+      unsigned got;
+      take(q, start, got, st);
+      if (threadIdx.x < C) peer_store(&s_got, threadIdx.x, got);
+    }
+    rung_sync<C>();
+    slot = s_got;
+    rung_sync<C>();
+    return slot != 0xFFFFFFFFu;
+  }
+}
+
 // R 5.6's point-to-plane rungs r_lo..r_hi-1 of the four per (pair, start)
 // (ladder.rs:142-161): from the item's start pose when r_lo is 0, else from
-// its rung r_lo - 1. With skip_partial, items an early rejection left partial
-// are passed over.
-template <class H, int MINB>
-__global__ void __launch_bounds__(ICP_BLOCK, MINB) k_ladder(const PairView *pairs,
+// its rung r_lo - 1, on one block of 128 G threads or a cluster of C of them per
+// item. With skip_partial, items an early rejection left partial are passed over.
+template <class H, int G, int C, int MINB>
+__global__ void __launch_bounds__(ICP_BLOCK *G, MINB) k_ladder(const PairView *pairs,
                                                       const sherd_work_item *items, QueueCtl q,
-                                                      H *hints, size_t hint_stride,
+                                                      IcpMemory<H> mem, size_t stride,
                                                       sherd_candidate *out, int r_lo, int r_hi,
                                                       int skip_partial, uint32_t *status) {
-  __shared__ IcpShared sh;
+  IcpBlock<G, C> &b = rung_memory<G, C>();
   uint32_t st = 0;
-  H *hint = hints + hint_stride * blockIdx.x;
+  const IcpMemory<H> mine = memory_slot(mem, blockIdx.x / C, stride);
   unsigned long long start = global_ns();
   unsigned it;
-  while (take(q, start, it, st)) {
+  while (take_shared<C>(q, start, it, st)) {
     const sherd_work_item &w = items[it];
     const PairView &pr = pairs[w.pair];
     sherd_candidate *c = out + it;
-    if (skip_partial && c->scores.partial) continue;  // the same for the whole block
+    if (skip_partial && c->scores.partial) continue;  // the same for every block of the item
     if (threadIdx.x < 16)
-      sh.t[threadIdx.x] = r_lo == 0 ? w.init[threadIdx.x] : c->rungs[r_lo - 1].transform[threadIdx.x];
-    if (threadIdx.x == 0 && r_lo == 0) {
+      b.s.t[threadIdx.x] = r_lo == 0 ? w.init[threadIdx.x] : c->rungs[r_lo - 1].transform[threadIdx.x];
+    if (threadIdx.x == 0 && cta_rank<C>() == 0 && r_lo == 0) {
       c->pair = w.pair;
       c->start = w.start;
     }
     __syncthreads();
     const double k[4] = {0.2, 0.08, 0.08, 0.04};
     for (int r = r_lo; r < r_hi; ++r) {
-      double distance = k[r] * pr.sc.t * pr.sc.icp;
+      const double distance = k[r] * pr.sc.t * pr.sc.icp;
       // Rungs 1 and 3 follow a rung over the same clouds (0 and 2): when that
-      // rung ran in this launch, its matches are this block's hints.
+      // rung ran in this launch, its matches still stand.
       const bool keep = (r & 1) && r > r_lo;
-      if (r < 2)
-        icp_rung_block(pr.reg_src, pr.n_reg, pr.reg_tgt, distance, 30, sh, hint, &c->rungs[r], st,
-                       false, keep);
-      else
-        icp_rung_block(pr.frac_src, pr.n_frac, pr.frac_tgt, distance, 30, sh, hint, &c->rungs[r],
-                       st, false, keep);
+      const bool reg = r < 2;
+      icp_rung_block<G, C>(reg ? pr.reg_src : pr.frac_src, reg ? pr.n_reg : pr.n_frac,
+                           reg ? pr.reg_tgt : pr.frac_tgt, distance, 30, b, mine,
+                           &c->rungs[r], st, false, keep);
     }
   }
   if (st) atomicOr(status, st);

@@ -116,6 +116,7 @@ __global__ void k_place_fused(const double *p, uint32_t n, Pose16 t, int rotate_
 
 struct WideState {
   double t[16];     // the pose of the next pass
+  double tp[16];    // the pose of the pass before it
   double fit, rmse; // the last pass's
   uint32_t pass;    // passes run so far in this rung
   uint32_t done;
@@ -124,7 +125,7 @@ struct WideState {
 
 // Starts a rung at `init` (16 doubles on the device).
 __global__ void k_wide_reset(WideState *s, const double *init) {
-  if (threadIdx.x < 16) s->t[threadIdx.x] = init[threadIdx.x];
+  if (threadIdx.x < 16) s->t[threadIdx.x] = s->tp[threadIdx.x] = init[threadIdx.x];
   if (threadIdx.x == 0) {
     s->fit = 0.0;
     s->rmse = 0.0;
@@ -134,16 +135,17 @@ __global__ void k_wide_reset(WideState *s, const double *init) {
   }
 }
 
-// icp::register's control after a pass (icp.rs:308-356), thread 0 of the last
-// block, with the pass's sums in sh.sums: after the first pass only the
-// initial fitness and rmse are kept; after pass p >= 1 the rung ends when both
-// moved by less than 1e-6 or p reaches max_iter; otherwise the point-to-plane
-// update of these sums moves the pose.
-__device__ __noinline__ void wide_control(const double *sums, uint32_t ns, int max_iter,
+// icp::register's control after a pass (icp.rs:308-356), the first warp of the
+// last block, with the pass's sums in sh.sums and its pose in sh.t: after the
+// first pass only the initial fitness and rmse are kept; after pass p >= 1 the
+// rung ends when both moved by less than 1e-6 or p reaches max_iter; otherwise
+// the point-to-plane update of these sums moves the pose.
+__device__ __noinline__ void wide_control(IcpShared &sh, uint32_t ns, int max_iter,
                                           WideState *state, sherd_registration *out) {
+  const int lane = threadIdx.x;
   double fit, rmse;
-  fit_rmse(sums, ns, fit, rmse);
-  uint32_t pass = state->pass;
+  fit_rmse(sh.sums, ns, fit, rmse);
+  const uint32_t pass = state->pass;
   bool converged = false, finish;
   if (pass == 0) {
     finish = max_iter <= 0;
@@ -151,22 +153,29 @@ __device__ __noinline__ void wide_control(const double *sums, uint32_t ns, int m
     converged = fabs(fit - state->fit) < 1e-6 && fabs(rmse - state->rmse) < 1e-6;
     finish = converged || int(pass) >= max_iter;
   }
-  state->fit = fit;
-  state->rmse = rmse;
-  state->pass = pass + 1;
+  __syncwarp();
+  if (lane == 0) {
+    state->fit = fit;
+    state->rmse = rmse;
+    state->pass = pass + 1;
+  }
   if (finish) {
-    for (int k = 0; k < 16; ++k) out->transform[k] = state->t[k];
-    out->fitness = fit;
-    out->inlier_rmse = rmse;
-    out->correspondences = (unsigned long long)sums[0];
-    out->iterations = pass;
-    out->converged = converged ? 1u : 0u;
-    state->done = 1;
+    if (lane < 16) out->transform[lane] = sh.t[lane];
+    if (lane == 0) {
+      out->fitness = fit;
+      out->inlier_rmse = rmse;
+      out->correspondences = (unsigned long long)sh.sums[0];
+      out->iterations = pass;
+      out->converged = converged ? 1u : 0u;
+      state->done = 1;
+    }
     return;
   }
-  double u[16];
-  plane_update(sums, true, u);
-  matmul4(u, state->t, state->t);
+  plane_step(sh.sums, true, sh.t, sh);
+  if (lane < 16) {
+    state->t[lane] = sh.t[lane];
+    state->tp[lane] = sh.tp[lane];
+  }
 }
 
 // One pass: block b over its slice [b chunk, (b + 1) chunk) of the source,
@@ -176,19 +185,25 @@ __device__ __noinline__ void wide_control(const double *sums, uint32_t ns, int m
 // depend on which block came last, and runs the rung's control. Every block
 // reads the state before it takes its ticket and only the last one writes it,
 // so the state is the same for the whole pass. No block waits for another.
-__global__ void __launch_bounds__(ICP_BLOCK, 4)
+__global__ void __launch_bounds__(ICP_BLOCK * 2, 2)
     k_wide_pass(const double4 *src, uint32_t ns, CloudView tgt, double distance, int max_iter,
-                WideState *state, int *hints, uint32_t chunk, double *partials,
+                WideState *state, IcpMemory<int> mem, uint32_t chunk, double *partials,
                 sherd_registration *out, uint32_t *status) {
-  __shared__ IcpShared sh;
+  IcpBlock<2, 1> &b = rung_memory<2, 1>();
   __shared__ uint32_t last;
+  IcpShared &sh = b.s;
   if (state->done) return;  // the same value for every block of the pass
   uint32_t st = 0;
-  if (threadIdx.x < 16) sh.t[threadIdx.x] = state->t[threadIdx.x];
+  if (threadIdx.x < 16) {
+    sh.t[threadIdx.x] = state->t[threadIdx.x];
+    sh.tp[threadIdx.x] = state->tp[threadIdx.x];
+  }
+  const bool fresh = state->pass == 0;
   __syncthreads();
   uint32_t lo = min(ns, blockIdx.x * chunk);
   uint32_t hi = min(ns, lo + chunk);
-  icp_pass(src + lo, hi - lo, tgt, distance * distance, distance > 0.0, sh, hints + lo, st);
+  const IcpMemory<int> mine = {mem.hint + lo, mem.slack + lo, nullptr, nullptr};
+  icp_pass<2, 1>(src + lo, hi - lo, tgt, distance * distance, distance > 0.0, b, mine, fresh, st);
   if (st) atomicOr(status, st);
   if (threadIdx.x < ICP_SUMS) partials[size_t(blockIdx.x) * ICP_SUMS + threadIdx.x] = sh.sums[threadIdx.x];
   __threadfence();
@@ -198,17 +213,15 @@ __global__ void __launch_bounds__(ICP_BLOCK, 4)
   if (!last) return;
   __threadfence();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int k = warp; k < ICP_SUMS; k += ICP_BLOCK / 32) {
+  for (int k = warp; k < ICP_SUMS; k += 8) {
     double v = 0.0;
     for (uint32_t b = lane; b < gridDim.x; b += 32u) v += __ldcg(partials + size_t(b) * ICP_SUMS + k);
     for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if (lane == 0) sh.sums[k] = v;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    state->ticket = 0;
-    wide_control(sh.sums, ns, max_iter, state, out);
-  }
+  if (threadIdx.x == 0) state->ticket = 0;
+  if (threadIdx.x < 32) wide_control(sh, ns, max_iter, state, out);
 }
 
 }  // namespace sherd

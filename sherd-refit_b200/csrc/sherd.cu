@@ -84,32 +84,42 @@ struct CtxLock {
   ~CtxLock() { t_alloc_ctx = prev; }
 };
 
-// Working memory of sherd_icp_rung_noalloc: each source point's last match, for
-// every candidate of one call. A file-scope device array, so that entry point
-// never allocates; every GPU that loads the library holds it until exit.
+// Working memory of sherd_icp_rung_noalloc: each source point's last match and
+// how far it stands (icp_match), for every candidate of one call. File-scope
+// device arrays, so that entry point never allocates; every GPU that loads the
+// library holds them until exit.
 static __device__ __align__(256) int g_noalloc_hints[SHERD_NOALLOC_CAPACITY];
+static __device__ __align__(256) float g_noalloc_slacks[SHERD_NOALLOC_CAPACITY];
+// Chunks of 32 points; a call with more of them does without (IcpMemory).
+constexpr uint32_t NOALLOC_CHUNKS = SHERD_NOALLOC_CAPACITY / 16;
+static __device__ __align__(256) IcpChunk g_noalloc_chunks[NOALLOC_CHUNKS];
+static __device__ __align__(256) float4 g_noalloc_balls[NOALLOC_CHUNKS];
 
 namespace {
 
 thread_local std::map<const sherd_ctx *, std::string> t_errors;
 
-// The device address of g_noalloc_hints, looked up once per device with that
-// device current (host code cannot use the symbol itself as an address).
+// The device addresses of those arrays, looked up once per device with that
+// device current (host code cannot use a symbol itself as an address).
 std::mutex g_symbol_mu;
-std::map<int, int *> g_noalloc_address;
+std::map<int, IcpMemory<int>> g_noalloc_address;
 
-cudaError_t noalloc_address(int device, int **out) {
+cudaError_t noalloc_address(int device, IcpMemory<int> *out) {
   std::lock_guard<std::mutex> lock(g_symbol_mu);
   auto it = g_noalloc_address.find(device);
   if (it != g_noalloc_address.end()) {
     *out = it->second;
     return cudaSuccess;
   }
-  void *p = nullptr;
-  cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_hints);
+  void *h = nullptr, *s = nullptr, *c = nullptr, *b = nullptr;
+  cudaError_t e = cudaGetSymbolAddress(&h, g_noalloc_hints);
+  if (e == cudaSuccess) e = cudaGetSymbolAddress(&s, g_noalloc_slacks);
+  if (e == cudaSuccess) e = cudaGetSymbolAddress(&c, g_noalloc_chunks);
+  if (e == cudaSuccess) e = cudaGetSymbolAddress(&b, g_noalloc_balls);
   if (e != cudaSuccess) return e;
-  g_noalloc_address[device] = static_cast<int *>(p);
-  *out = static_cast<int *>(p);
+  *out = {static_cast<int *>(h), static_cast<float *>(s), static_cast<IcpChunk *>(c),
+          static_cast<float4 *>(b)};
+  g_noalloc_address[device] = *out;
   return cudaSuccess;
 }
 
@@ -174,6 +184,25 @@ struct DBuf {  // owning device buffer
       return e;
     }
     return cudaMalloc(&p, count * sizeof(T));
+  }
+};
+
+// A rung's memory (IcpMemory) for `slots` items of up to n points.
+struct RungBuffers {
+  DBuf<unsigned char> hints;
+  DBuf<float> slacks;
+  DBuf<IcpChunk> chunks;
+  DBuf<float4> balls;
+  cudaError_t alloc(size_t n, size_t slots, size_t hint_size) {
+    cudaError_t e = hints.alloc(std::max<size_t>(1, n * slots) * hint_size);
+    if (e == cudaSuccess) e = slacks.alloc(std::max<size_t>(1, n * slots));
+    if (e == cudaSuccess) e = chunks.alloc(std::max<size_t>(1, (n + 31) / 32 * slots));
+    if (e == cudaSuccess) e = balls.alloc(std::max<size_t>(1, (n + 31) / 32 * slots));
+    return e;
+  }
+  template <class H>
+  IcpMemory<H> view() const {
+    return {reinterpret_cast<H *>(hints.p), slacks.p, chunks.p, balls.p};
   }
 };
 
@@ -583,6 +612,60 @@ int radix_sort_pairs(sherd_ctx *ctx, const K *kin, K *kout, const V *vin, V *vou
                                      ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   return SHERD_OK;
+}
+
+// The block and cluster shape of a rung: G groups of 128 threads, C blocks.
+struct RungForm {
+  int g, c;
+};
+
+// The form for k candidates of `points` points. With fewer candidates than SMs a
+// rung's time is the length of its passes, so a candidate gets as many blocks of
+// 512 threads (a cluster of up to 8) as there are SMs for, while a block has 256
+// points to itself: ten starts of 6000 points took 24.1 ms on a block each and
+// take 2.0 ms on clusters of 8, ten whole ladders 50.1 and 3.4 ms. With many, the
+// 256-thread form is the faster one (its searches need no block-wide barrier): a
+// pot's 1792 ladders take 51.7 ms on it and 71 ms on 512-thread blocks.
+RungForm rung_form(const sherd_ctx *ctx, uint64_t k, uint64_t points) {
+  const uint64_t sms = uint64_t(std::max(ctx->sm_count, 1));
+  for (int c = 8; c > 1; c /= 2)
+    if (k * uint64_t(c) <= sms && points >= 512u * uint64_t(c) / 2u) return {4, c};
+  return k <= 2 * sms && points > 256 ? RungForm{4, 1} : RungForm{2, 1};
+}
+
+template <int G, int C, class... Args>
+cudaError_t launch_cluster(void (*kernel)(Args...), unsigned clusters, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(clusters * C);
+  cfg.blockDim = dim3(ICP_BLOCK * G);
+  cfg.stream = s;
+  if (C > 1) {
+    cfg.dynamicSmemBytes = sizeof(IcpBlock<G, C>);
+    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void *>(kernel),
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(cfg.dynamicSmemBytes));
+    if (e != cudaSuccess) return e;
+  }
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = C;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = C > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+cudaError_t launch_rung(sherd_ctx *ctx, const double4 *src, uint32_t ns, const CloudView &tgt,
+                        const double *inits, uint32_t k, sherd_icp_options opt,
+                        const IcpMemory<int> &mem, sherd_registration *out) {
+  const RungForm f = rung_form(ctx, k, ns);
+  cudaStream_t s = ctx->stream;
+  uint32_t *st = ctx->d_status;
+  if (f.c == 8) return launch_cluster<4, 8>(k_icp_rung<4, 8>, k, s, src, ns, tgt, inits, opt, mem, out, st);
+  if (f.c == 4) return launch_cluster<4, 4>(k_icp_rung<4, 4>, k, s, src, ns, tgt, inits, opt, mem, out, st);
+  if (f.c == 2) return launch_cluster<4, 2>(k_icp_rung<4, 2>, k, s, src, ns, tgt, inits, opt, mem, out, st);
+  if (f.g == 4) return launch_cluster<4, 1>(k_icp_rung<4, 1>, k, s, src, ns, tgt, inits, opt, mem, out, st);
+  return launch_cluster<2, 1>(k_icp_rung<2, 1>, k, s, src, ns, tgt, inits, opt, mem, out, st);
 }
 
 bool has_nan(const double *p, size_t n) {
@@ -1217,8 +1300,8 @@ int sherd_icp_rung(sherd_ctx *ctx, const double *source, uint32_t n_source, cons
   sherd_cloud src;
   DBuf<double> di;
   DBuf<sherd_registration> dout;
-  DBuf<int> hints;
-  CK(hints.alloc(std::max<size_t>(1, size_t(n_source) * k)));
+  RungBuffers mem;
+  CK(mem.alloc(n_source, k, sizeof(int)));
   if (n_source) {
     if (has_nan(source, size_t(3) * n_source)) return fail(ctx, SHERD_E_INVALID, "non-finite source point");
     rc = cloud_build(ctx, source, nullptr, n_source, &src);
@@ -1228,9 +1311,8 @@ int sherd_icp_rung(sherd_ctx *ctx, const double *source, uint32_t n_source, cons
   CK(dout.alloc(k));
   CK(cudaMemsetAsync(ctx->d_status, 0, 4, ctx->stream));
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
-  k_icp_rung<<<k, ICP_BLOCK, 0, ctx->stream>>>(n_source ? src.pts.p : nullptr, n_source, target->view,
-                                               di.p, options, hints.p, dout.p, ctx->d_status);
-  CK(cudaGetLastError());
+  CK(launch_rung(ctx, n_source ? src.pts.p : nullptr, n_source, target->view, di.p, k, options,
+                 mem.view<int>(), dout.p));
   CK(cudaMemcpyAsync(out, dout.p, sizeof(sherd_registration) * k, cudaMemcpyDeviceToHost, ctx->stream));
   return finish(ctx, "icp_rung", k, true);
 }
@@ -1272,14 +1354,13 @@ int sherd_icp_rung_noalloc(sherd_ctx *ctx, const double *source, uint32_t n_sour
   CtxLock lock(ctx);
   int rc = begin(ctx);  // makes the context's device current
   if (rc) return rc;
-  // The first call on a device looks the array's address up; that call should
+  // The first call on a device looks the arrays' addresses up; that call should
   // come before any stream capture on the device.
-  int *hints = nullptr;
-  CK(noalloc_address(ctx->device, &hints));
-  k_icp_rung<<<k, ICP_BLOCK, 0, ctx->stream>>>(reinterpret_cast<const double4 *>(source), n_source,
-                                               target->view, inits, options, hints, out,
-                                               ctx->d_status);
-  CK(cudaGetLastError());
+  IcpMemory<int> mem;
+  CK(noalloc_address(ctx->device, &mem));
+  if (uint64_t(k) * ((n_source + 31u) / 32u) > NOALLOC_CHUNKS) mem.chunks = nullptr, mem.balls = nullptr;
+  CK(launch_rung(ctx, reinterpret_cast<const double4 *>(source), n_source, target->view, inits, k,
+                 options, mem, out));
   return finish(ctx, "icp_rung_noalloc", k, true);
 }
 
@@ -1515,36 +1596,42 @@ struct sherd_batch {
   DBuf<sherd_candidate> dc;
   DBuf<uint32_t> dorder;
   DBuf<unsigned> heads, scratch;
-  // Per ladder CTA, each source point's last match: 16 bits when every target
-  // of the batch has fewer than 65535 points, else an int.
-  DBuf<unsigned char> hints;
+  // Per item in flight, each source point's last match (16 bits when every target
+  // of the batch has fewer than 65535 points, else an int) and how far it stands.
+  RungBuffers mem;
   bool hint16 = true;
   size_t hint_stride = 1;
-  // Launches k_ladder variant v (rungs r_lo..r_hi-1) with the batch's hint
-  // width, its CTAs using the hint slots from slot0 on.
-  template <class H, int MINB>
-  void ladder_as(unsigned grid, QueueCtl q, cudaStream_t s, int r_lo, int r_hi, int skip_partial,
-                 size_t slot0) {
-    H *h = reinterpret_cast<H *>(hints.p) + slot0 * hint_stride;
-    k_ladder<H, MINB><<<grid, ICP_BLOCK, 0, s>>>(dv.p, di.p, q, h, hint_stride, dc.p, r_lo, r_hi,
-                                                 skip_partial, ctx->d_status);
+  // Launches k_ladder (rungs r_lo..r_hi-1) for `n` items in flight, on the slots
+  // from slot0 on: variant v of the 256-thread blocks, or the wide form `wide`
+  // (clusters of so many 512-thread blocks; 0: none), whose hints are always ints.
+  template <class H, int G, int C, int MINB>
+  cudaError_t ladder_as(unsigned n, QueueCtl q, cudaStream_t s, int r_lo, int r_hi,
+                        int skip_partial, size_t slot0) {
+    return launch_cluster<G, C>(k_ladder<H, G, C, MINB>, n, s, (const PairView *)dv.p,
+                                (const sherd_work_item *)di.p, q,
+                                memory_slot(mem.view<H>(), slot0, hint_stride), hint_stride, dc.p,
+                                r_lo, r_hi, skip_partial, ctx->d_status);
   }
   template <class H>
-  void ladder_h(int v, unsigned grid, QueueCtl q, cudaStream_t s, int r_lo, int r_hi,
-                int skip_partial, size_t slot0) {
-    if (v == 0)
-      ladder_as<H, LADDER_MINB[0]>(grid, q, s, r_lo, r_hi, skip_partial, slot0);
-    else if (v == 1)
-      ladder_as<H, LADDER_MINB[1]>(grid, q, s, r_lo, r_hi, skip_partial, slot0);
-    else
-      ladder_as<H, LADDER_MINB[2]>(grid, q, s, r_lo, r_hi, skip_partial, slot0);
+  cudaError_t ladder_h(int v, unsigned n, QueueCtl q, cudaStream_t s, int r_lo, int r_hi,
+                       int skip_partial, size_t slot0) {
+    if (v == 0) return ladder_as<H, 2, 1, LADDER_MINB[0]>(n, q, s, r_lo, r_hi, skip_partial, slot0);
+    if (v == 1) return ladder_as<H, 2, 1, LADDER_MINB[1]>(n, q, s, r_lo, r_hi, skip_partial, slot0);
+    return ladder_as<H, 2, 1, LADDER_MINB[2]>(n, q, s, r_lo, r_hi, skip_partial, slot0);
   }
-  void ladder(unsigned grid, QueueCtl q, cudaStream_t s, int r_lo, int r_hi, int skip_partial,
-              int v = LADDER_DEFAULT, size_t slot0 = 0) {
-    if (hint16)
-      ladder_h<uint16_t>(v, grid, q, s, r_lo, r_hi, skip_partial, slot0);
-    else
-      ladder_h<int>(v, grid, q, s, r_lo, r_hi, skip_partial, slot0);
+  cudaError_t ladder(unsigned n, QueueCtl q, cudaStream_t s, int r_lo, int r_hi, int skip_partial,
+                     int v, size_t slot0, int wide) {
+    if (wide == 8) return ladder_as<int, 4, 8, 1>(n, q, s, r_lo, r_hi, skip_partial, slot0);
+    if (wide == 4) return ladder_as<int, 4, 4, 1>(n, q, s, r_lo, r_hi, skip_partial, slot0);
+    if (wide == 2) return ladder_as<int, 4, 2, 1>(n, q, s, r_lo, r_hi, skip_partial, slot0);
+    if (wide == 1) return ladder_as<int, 4, 1, 2>(n, q, s, r_lo, r_hi, skip_partial, slot0);
+    return hint16 ? ladder_h<uint16_t>(v, n, q, s, r_lo, r_hi, skip_partial, slot0)
+                  : ladder_h<int>(v, n, q, s, r_lo, r_hi, skip_partial, slot0);
+  }
+  // The wide form of a launch of n items, none in flight beside it (0: not wide).
+  int wide_of(uint64_t n) const {
+    const RungForm f = rung_form(ctx, n, hint_stride);
+    return f.g == 4 ? f.c : 0;
   }
   // The ladder's point-count buckets (largest moving clouds first): each is a
   // segment of the queue order, run by its own k_ladder variant (chosen by the
@@ -1553,9 +1640,12 @@ struct sherd_batch {
   uint32_t seg_first[BUCKETS] = {}, seg_count[BUCKETS] = {};
   int variant[BUCKETS] = {LADDER_DEFAULT, LADDER_DEFAULT, LADDER_DEFAULT};
   size_t slot0[BUCKETS] = {};
+  int wide[BUCKETS] = {};
   int occ[LADDER_VARIANTS] = {};  // resident k_ladder CTAs per SM of each variant
   DBuf<unsigned> lheads;          // one queue head per bucket
   unsigned bucket_grid(int b) const {
+    if (wide[b] == 1) return std::max(1u, std::min<unsigned>(2u * ctx->sm_count, seg_count[b]));
+    if (wide[b]) return seg_count[b];
     return std::max(1u, std::min<unsigned>(unsigned(std::max(1, occ[variant[b]]) * ctx->sm_count),
                                            seg_count[b]));
   }
@@ -1604,8 +1694,8 @@ int ladder_stage(sherd_batch *b, cudaStream_t s, unsigned *heads, const uint32_t
   unsigned long long budget = (unsigned long long)ctx->timeout_ms * 1000000ULL;
   const bool early = b->early();
   QueueCtl q0{heads, order, n, ctx->abort_dev, budget};
-  b->ladder(grid, q0, s, 0, early ? 2 : 4, 0);
-  CK(cudaGetLastError());
+  const int wide = b->wide_of(n);
+  CK(b->ladder(grid, q0, s, 0, early ? 2 : 4, 0, LADDER_DEFAULT, 0, wide));
   if (early) {
     QueueCtl q1{heads + 2, order, n, ctx->abort_dev, budget};
     k_verify_items<<<std::min<unsigned>(b->grid_v, n), VER_BLOCK, 0, s>>>(
@@ -1614,8 +1704,7 @@ int ladder_stage(sherd_batch *b, cudaStream_t s, unsigned *heads, const uint32_t
     k_early_mark<<<blocks_for(n), 256, 0, s>>>(b->dc.p, order, n, b->params.early_reject_tight);
     CK(cudaGetLastError());
     QueueCtl q2{heads + 3, order, n, ctx->abort_dev, budget};
-    b->ladder(grid, q2, s, 2, 4, 1);
-    CK(cudaGetLastError());
+    CK(b->ladder(grid, q2, s, 2, 4, 1, LADDER_DEFAULT, 0, wide));
   }
   return SHERD_OK;
 }
@@ -1640,8 +1729,7 @@ int launch_ladder(sherd_batch *b, cudaStream_t s) {
     cudaStream_t on = bk == 0 ? s : ctx->side[bk - 1];
     QueueCtl q{b->lheads.p + bk, b->dorder.p + b->seg_first[bk], b->seg_count[bk], ctx->abort_dev,
                budget};
-    b->ladder(b->bucket_grid(bk), q, on, 0, 4, 0, b->variant[bk], b->slot0[bk]);
-    CK(cudaGetLastError());
+    CK(b->ladder(b->bucket_grid(bk), q, on, 0, 4, 0, b->variant[bk], b->slot0[bk], b->wide[bk]));
   }
   for (int k = 0; k < 2; ++k) {
     CK(cudaEventRecord(ctx->join_ev[k], ctx->side[k]));
@@ -1681,8 +1769,7 @@ int tune_ladder(sherd_batch *b) {
       QueueCtl q{b->lheads.p + bk, b->dorder.p + b->seg_first[bk], need, ctx->abort_dev, 0ull};
       CK(cudaMemsetAsync(b->lheads.p + bk, 0, sizeof(unsigned), s));
       CK(cudaEventRecord(ctx->ev0, s));
-      b->ladder(grid, q, s, 0, 4, 0, run, b->slot0[bk]);
-      CK(cudaGetLastError());
+      CK(b->ladder(grid, q, s, 0, 4, 0, run, b->slot0[bk], 0));
       CK(cudaEventRecord(ctx->ev1, s));
       CK(cudaStreamSynchronize(s));
       float ms = 0.0f;
@@ -1852,14 +1939,15 @@ int batch_create(sherd_ctx *ctx, sherd_pair *const *pairs, uint32_t n_pairs,
   CK(cudaMemsetAsync(b->dc.p, 0, sizeof(sherd_candidate) * n_items, ctx->stream));
   CK(b->heads.alloc(sherd_batch::HEADS * size_t(std::max<uint32_t>(n_pairs, 1))));
   int occ_v = 0;
+  const int threads = 2 * ICP_BLOCK;
   if (b->hint16) {
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[0], k_ladder<uint16_t, LADDER_MINB[0]>, ICP_BLOCK, 0));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[1], k_ladder<uint16_t, LADDER_MINB[1]>, ICP_BLOCK, 0));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[2], k_ladder<uint16_t, LADDER_MINB[2]>, ICP_BLOCK, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[0], k_ladder<uint16_t, 2, 1, LADDER_MINB[0]>, threads, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[1], k_ladder<uint16_t, 2, 1, LADDER_MINB[1]>, threads, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[2], k_ladder<uint16_t, 2, 1, LADDER_MINB[2]>, threads, 0));
   } else {
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[0], k_ladder<int, LADDER_MINB[0]>, ICP_BLOCK, 0));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[1], k_ladder<int, LADDER_MINB[1]>, ICP_BLOCK, 0));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[2], k_ladder<int, LADDER_MINB[2]>, ICP_BLOCK, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[0], k_ladder<int, 2, 1, LADDER_MINB[0]>, threads, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[1], k_ladder<int, 2, 1, LADDER_MINB[1]>, threads, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[2], k_ladder<int, 2, 1, LADDER_MINB[2]>, threads, 0));
   }
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_v, k_verify_items, VER_BLOCK, 0));
   b->grid_l = unsigned(std::max(1, b->occ[LADDER_DEFAULT]) * ctx->sm_count);
@@ -1903,9 +1991,9 @@ int batch_create(sherd_ctx *ctx, sherd_pair *const *pairs, uint32_t n_pairs,
     b->grid_m = unsigned(std::max(1, occ_m) * ctx->sm_count);
   }
   b->hint_stride = (b->hint_stride + 63) / 64 * 64;
-  // The plain schedule launches one CTA per item of a pair, so it needs as many
-  // hint slots as the largest pair has items.
-  size_t slots = b->grid_l;
+  // The plain schedule launches one block or cluster per item of a pair, so it
+  // needs as many hint slots as the largest pair has items.
+  size_t slots = std::max<size_t>(b->grid_l, 2 * size_t(ctx->sm_count));
   for (uint32_t c : b->pair_count) slots = std::max<size_t>(slots, c);
   if (sched == SHERD_SCHED_BATCHED) {
     // The buckets' launches run side by side, each on its own slice of slots,
@@ -1913,14 +2001,19 @@ int batch_create(sherd_ctx *ctx, sherd_pair *const *pairs, uint32_t n_pairs,
     int max_occ = 1;
     for (int v = 0; v < LADDER_VARIANTS; ++v) max_occ = std::max(max_occ, b->occ[v]);
     size_t acc = 0;
+    // Few items in all: wide blocks, chosen by the items of all the buckets.
+    const int wide = b->wide_of(n_items);
     for (int bk = 0; bk < sherd_batch::BUCKETS; ++bk) {
       b->slot0[bk] = acc;
-      acc += std::min<size_t>(size_t(max_occ) * ctx->sm_count, b->seg_count[bk]);
+      b->wide[bk] = wide;
+      acc += std::min<size_t>(wide ? size_t(n_items) : size_t(max_occ) * ctx->sm_count, b->seg_count[bk]);
     }
     slots = std::max(slots, acc);
     CK(b->lheads.alloc(sherd_batch::BUCKETS));
   }
-  CK(b->hints.alloc(slots * b->hint_stride * (b->hint16 ? sizeof(uint16_t) : sizeof(int))));
+  // Ints wherever a wide form may run on them (it has no 16-bit variant).
+  const bool ints = !b->hint16 || b->sched == SHERD_SCHED_PLAIN || b->early() || b->wide[0];
+  CK(b->mem.alloc(b->hint_stride, slots, ints ? sizeof(int) : sizeof(uint16_t)));
   for (cudaEvent_t &e : b->ev) CK(cudaEventCreate(&e));
   CK(cudaStreamSynchronize(ctx->stream));
   if (sched == SHERD_SCHED_BATCHED) {
@@ -2612,11 +2705,11 @@ int sherd_refine_join(sherd_ctx *ctx, const double *source, uint32_t n_source,
       std::max(1u, std::min<uint32_t>((ns + 255u) / 256u, 4u * uint32_t(std::max(ctx->sm_count, 1))));
   const uint32_t chunk = (ns + blocks - 1u) / blocks;
   DBuf<double> partials, identity;
-  DBuf<int> hints;
+  RungBuffers mem;
   DBuf<WideState> state;
   DBuf<sherd_registration> dout;
   CK(partials.alloc(size_t(blocks) * ICP_SUMS));
-  CK(hints.alloc(ns));
+  CK(mem.alloc(ns, 1, sizeof(int)));
   CK(state.alloc(1));
   CK(dout.alloc(2));
   static const double kIdentity[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1};
@@ -2641,14 +2734,13 @@ int sherd_refine_join(sherd_ctx *ctx, const double *source, uint32_t n_source,
   uint32_t done = 0;
   size_t launched = 0;
   for (int r = 0; r < 2; ++r) {
-    CK(cudaMemsetAsync(hints.p, 0xFF, sizeof(int) * size_t(ns), s));  // no match yet: -1
     k_wide_reset<<<1, 32, 0, s>>>(state.p, r == 0 ? identity.p : first_pose);
     // max_iteration + 1 passes at most; the state says when the rung ended
     // sooner, looked at every 16 passes.
     for (int64_t pass = 0; pass <= int64_t(max_iteration); ++pass) {
-      k_wide_pass<<<blocks, ICP_BLOCK, 0, s>>>(src.pts.p, ns, tgt.view, dist[r], max_iteration,
-                                               state.p, hints.p, chunk, partials.p, dout.p + r,
-                                               ctx->d_status);
+      k_wide_pass<<<blocks, 2 * ICP_BLOCK, 0, s>>>(src.pts.p, ns, tgt.view, dist[r], max_iteration,
+                                                   state.p, mem.view<int>(), chunk, partials.p,
+                                                   dout.p + r, ctx->d_status);
       CK(cudaGetLastError());
       ++launched;
       if (pass % 16 == 15 && pass < int64_t(max_iteration)) {

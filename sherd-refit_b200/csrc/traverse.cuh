@@ -198,39 +198,32 @@ __device__ __forceinline__ float box_dist2(const float *lo, const float *hi, con
 }
 
 // A walk over a 4-wide tree (WNode) with the binary tree's own boxes: at each
-// node the children in ascending box distance, leaves scored first (nearest
-// first, each against the bound as it stands), then the nearest node taken
-// and the others stacked with the nearest on top. Every leaf whose box lies
-// within the bound is scored, whatever the order, so a search's answer is the
-// binary walk's. `bound2()` is the squared bound on box distances; `leaf`
-// returns true to end the walk. (Point clouds only: on the mesh trees the
-// closest-face walks measured 4 % faster in the minimum pass but the inside
-// pass, whose kernel the wider walk costs registers, 50 % slower.)
-template <class Leaf, class Bound2>
+// node the leaves within the bound are scored, then the nearest node is taken
+// and the others are stacked. Every leaf whose box lies within the bound is
+// scored, whatever the order, so a search's answer is the binary walk's.
+// `bound2()` is the squared bound on box distances, `leaf(first, count)` scores a
+// leaf, `left(k)` is told the squared box distance of what the walk does not
+// enter. (Point clouds only: on the mesh trees the closest-face walks measured
+// 4 % faster in the minimum pass but the inside pass, whose kernel the wider
+// walk costs registers, 50 % slower.)
+//
+// The walk is bound by its instructions: the lanes of a warp are at different
+// nodes, and a branch taken by one lane costs all of them. The leaves of a node
+// are therefore scored by one loop over a mask of its children, as often as
+// the lane with most leaves needs (a branch per child ran the scoring code four
+// times a node), and the children are not sorted: with a good first bound
+// nearly all that is within it has to be scored in any order.
+template <class Leaf, class Bound2, class Left>
 __device__ __forceinline__ void wide_walk(const WNode *wide, const float *pc, uint32_t limit,
-                                          Leaf &&leaf, Bound2 &&bound2, uint32_t &status) {
+                                          Leaf &&leaf, Bound2 &&bound2, Left &&left,
+                                          uint32_t &status) {
   int stack_n[STACK];
   float stack_k[STACK];
   int sp = 0, node = 0;
   uint32_t visits = 0;
-  auto push = [&](int r, float k) {
-    if (sp < STACK) {
-      stack_n[sp] = r;
-      stack_k[sp++] = k;
-    } else {
-      status |= ST_STACK;
-    }
-  };
   auto bd = [&](float x0, float y0, float z0, float x1, float y1, float z1) {
     const float lo[3] = {x0, y0, z0}, hi[3] = {x1, y1, z1};
     return box_dist2(lo, hi, pc);
-  };
-  auto order = [](float &ka, int &ra, int &na, float &kb, int &rb, int &nb) {
-    if (kb < ka) {
-      float tk = ka; ka = kb; kb = tk;
-      int tr = ra; ra = rb; rb = tr;
-      int tn = na; na = nb; nb = tn;
-    }
   };
   for (;;) {
     if (++visits > limit) {
@@ -242,40 +235,63 @@ __device__ __forceinline__ void wide_walk(const WNode *wide, const float *pc, ui
     const float4 hx = __ldg(w + 3), hy = __ldg(w + 4), hz = __ldg(w + 5);
     const int4 rf = __ldg(reinterpret_cast<const int4 *>(w + 6));
     const int4 ct = __ldg(reinterpret_cast<const int4 *>(w + 7));
-    float k0 = bd(lx.x, ly.x, lz.x, hx.x, hy.x, hz.x), k1 = bd(lx.y, ly.y, lz.y, hx.y, hy.y, hz.y);
-    float k2 = bd(lx.z, ly.z, lz.z, hx.z, hy.z, hz.z), k3 = bd(lx.w, ly.w, lz.w, hx.w, hy.w, hz.w);
-    int r0 = rf.x, r1 = rf.y, r2 = rf.z, r3 = rf.w;
-    int n0 = ct.x, n1 = ct.y, n2 = ct.z, n3 = ct.w;
-    order(k0, r0, n0, k1, r1, n1);
-    order(k2, r2, n2, k3, r3, n3);
-    order(k0, r0, n0, k2, r2, n2);
-    order(k1, r1, n1, k3, r3, n3);
-    order(k1, r1, n1, k2, r2, n2);
-    if (n0 > 0 && k0 <= bound2() && leaf(r0, n0)) return;
-    if (n1 > 0 && k1 <= bound2() && leaf(r1, n1)) return;
-    if (n2 > 0 && k2 <= bound2() && leaf(r2, n2)) return;
-    if (n3 > 0 && k3 <= bound2() && leaf(r3, n3)) return;
-    const float b = bound2();
-    const bool i0 = n0 == 0 && k0 <= b, i1 = n1 == 0 && k1 <= b, i2 = n2 == 0 && k2 <= b,
-               i3 = n3 == 0 && k3 <= b;
-    const int first = i0 ? 0 : i1 ? 1 : i2 ? 2 : i3 ? 3 : 4;
-    if (i3 && first != 3) push(r3, k3);
-    if (i2 && first != 2) push(r2, k2);
-    if (i1 && first != 1) push(r1, k1);
-    if (first < 4) {
-      node = first == 0 ? r0 : first == 1 ? r1 : first == 2 ? r2 : r3;
-      continue;
+    const float k[4] = {bd(lx.x, ly.x, lz.x, hx.x, hy.x, hz.x), bd(lx.y, ly.y, lz.y, hx.y, hy.y, hz.y),
+                        bd(lx.z, ly.z, lz.z, hx.z, hy.z, hz.z), bd(lx.w, ly.w, lz.w, hx.w, hy.w, hz.w)};
+    const int r[4] = {rf.x, rf.y, rf.z, rf.w}, n[4] = {ct.x, ct.y, ct.z, ct.w};
+    float b = bound2();
+    unsigned leaves = 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) leaves |= n[c] > 0 && k[c] <= b ? 1u << c : 0u;
+    while (leaves) {
+      const int c = __ffs(leaves) - 1;
+      leaves &= leaves - 1u;
+      leaf(c < 2 ? (c == 0 ? r[0] : r[1]) : (c == 2 ? r[2] : r[3]),
+           c < 2 ? (c == 0 ? n[0] : n[1]) : (c == 2 ? n[2] : n[3]));
     }
-    bool more = false;
-    while (sp > 0) {
-      --sp;
-      if (stack_k[sp] <= bound2()) {
-        node = stack_n[sp];
-        more = true;
-        break;
+    float out = f_inf();  // the nearest child not entered
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (n[c] != 0 && !(k[c] <= b)) out = fminf(out, k[c]);
+    b = bound2();
+    float nearest = f_inf();
+    int next = -1;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (n[c] == 0) {
+        if (!(k[c] <= b)) {
+          out = fminf(out, k[c]);
+        } else {
+          // The nearer of this child and the one in hand goes on, the other is stacked.
+          const bool here = next < 0 || k[c] < nearest;
+          const int rs = here ? next : r[c];
+          const float ks = here ? nearest : k[c];
+          if (here) {
+            next = r[c];
+            nearest = k[c];
+          }
+          if (rs >= 0) {
+            if (sp < STACK) {
+              stack_n[sp] = rs;
+              stack_k[sp++] = ks;
+            } else {
+              status |= ST_STACK;
+            }
+          }
+        }
       }
+    left(out);
+    if (next < 0) {
+      while (sp > 0) {
+        --sp;
+        if (stack_k[sp] <= b) {
+          next = stack_n[sp];
+          break;
+        }
+        left(stack_k[sp]);
+      }
+      if (next < 0) return;
     }
-    if (!more) return;
+    node = next;
   }
 }
 
@@ -528,11 +544,7 @@ __device__ __noinline__ int nearest_within_sq(const CloudView &c, double qx, dou
   if (c.wide) {
     wide_walk(
         c.wide, qc, 2u * c.n + 64u,
-        [&](int first, int count) {
-          leaf(first, count);
-          return false;
-        },
-        bound2, status);
+        leaf, bound2, [](float) {}, status);
     return best_s;
   }
   for (;;) {
