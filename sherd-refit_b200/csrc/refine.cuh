@@ -178,6 +178,9 @@ __device__ __noinline__ void wide_control(IcpShared &sh, uint32_t ns, int max_it
   }
 }
 
+// Groups of 128 threads in a block of a wide pass.
+constexpr int WIDE_G = 4;
+
 // One pass: block b over its slice [b chunk, (b + 1) chunk) of the source,
 // its 29 sums written to partials[b]. The block that finishes last (a ticket
 // taken after a fence) adds the slices' sums, each sum by one warp over the
@@ -185,11 +188,11 @@ __device__ __noinline__ void wide_control(IcpShared &sh, uint32_t ns, int max_it
 // depend on which block came last, and runs the rung's control. Every block
 // reads the state before it takes its ticket and only the last one writes it,
 // so the state is the same for the whole pass. No block waits for another.
-__global__ void __launch_bounds__(ICP_BLOCK * 2, 2)
+__global__ void __launch_bounds__(ICP_BLOCK * WIDE_G, 4 / WIDE_G)
     k_wide_pass(const double4 *src, uint32_t ns, CloudView tgt, double distance, int max_iter,
                 WideState *state, IcpMemory<int> mem, uint32_t chunk, double *partials,
                 sherd_registration *out, uint32_t *status) {
-  IcpBlock<2, 1> &b = rung_memory<2, 1>();
+  IcpBlock<WIDE_G, 1> &b = rung_memory<WIDE_G, 1>();
   __shared__ uint32_t last;
   IcpShared &sh = b.s;
   if (state->done) return;  // the same value for every block of the pass
@@ -203,7 +206,7 @@ __global__ void __launch_bounds__(ICP_BLOCK * 2, 2)
   uint32_t lo = min(ns, blockIdx.x * chunk);
   uint32_t hi = min(ns, lo + chunk);
   const IcpMemory<int> mine = {mem.hint + lo, mem.slack + lo, nullptr, nullptr};
-  icp_pass<2, 1>(src + lo, hi - lo, tgt, distance * distance, distance > 0.0, b, mine, fresh, st);
+  icp_pass<WIDE_G, 1>(src + lo, hi - lo, tgt, distance * distance, distance > 0.0, b, mine, fresh, st);
   if (st) atomicOr(status, st);
   if (threadIdx.x < ICP_SUMS) partials[size_t(blockIdx.x) * ICP_SUMS + threadIdx.x] = sh.sums[threadIdx.x];
   __threadfence();
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(ICP_BLOCK * 2, 2)
   if (!last) return;
   __threadfence();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int k = warp; k < ICP_SUMS; k += 8) {
+  for (int k = warp; k < ICP_SUMS; k += 4 * WIDE_G) {
     double v = 0.0;
     for (uint32_t b = lane; b < gridDim.x; b += 32u) v += __ldcg(partials + size_t(b) * ICP_SUMS + k);
     for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);

@@ -2738,7 +2738,7 @@ int sherd_refine_join(sherd_ctx *ctx, const double *source, uint32_t n_source,
     // max_iteration + 1 passes at most; the state says when the rung ended
     // sooner, looked at every 16 passes.
     for (int64_t pass = 0; pass <= int64_t(max_iteration); ++pass) {
-      k_wide_pass<<<blocks, 2 * ICP_BLOCK, 0, s>>>(src.pts.p, ns, tgt.view, dist[r], max_iteration,
+      k_wide_pass<<<blocks, WIDE_G * ICP_BLOCK, 0, s>>>(src.pts.p, ns, tgt.view, dist[r], max_iteration,
                                                    state.p, mem.view<int>(), chunk, partials.p,
                                                    dout.p + r, ctx->d_status);
       CK(cudaGetLastError());
