@@ -364,11 +364,32 @@ constexpr int LADDER_MINB[LADDER_VARIANTS] = {3, 4, 5};
 // too few items to time).
 constexpr int LADDER_DEFAULT = 1;
 
+// How a running kernel hears of sherd_abort: the host's flag is mapped memory,
+// a read of it crosses the bus (about 0.8 us each, one after the other for the
+// whole device: a warp that polled it when it started made 4736 warps wait 3.8 ms
+// for their first chunk), so one thread at a time reads it, every POLL_NS, and
+// the rest read its copy on the device. The copy is cleared with the status word.
+struct StopCtl {
+  const uint32_t *host;       // host-mapped; non-zero asks the kernel to stop
+  uint32_t *seen;             // the device's copy
+  unsigned long long *polled; // when it was last refreshed (global_ns)
+};
+constexpr unsigned long long POLL_NS = 20000;
+
+__device__ __forceinline__ bool stop_asked(const StopCtl &c) {
+  if (*((volatile uint32_t *)c.seen)) return true;
+  const unsigned long long last = *((volatile unsigned long long *)c.polled), now = global_ns();
+  if (now - last < POLL_NS || atomicCAS(c.polled, last, now) != last) return false;
+  if (!*((volatile const uint32_t *)c.host)) return false;
+  *((volatile uint32_t *)c.seen) = 1u;
+  return true;
+}
+
 struct QueueCtl {
   unsigned *head;             // next queue position to take
   const uint32_t *order;      // item indices, most expensive first
   uint32_t n;                 // queue length
-  const uint32_t *abort_flag; // host-mapped; non-zero asks the kernel to stop
+  StopCtl stop;
   unsigned long long budget_ns;
 };
 
@@ -379,7 +400,7 @@ __device__ __forceinline__ bool take(const QueueCtl &q, unsigned long long start
   __shared__ unsigned s_item;
   if (threadIdx.x == 0) {
     unsigned item = 0xFFFFFFFFu;
-    if (q.abort_flag && *((volatile const uint32_t *)q.abort_flag)) {
+    if (q.stop.host && stop_asked(q.stop)) {
       st |= ST_ABORTED;
     } else if (q.budget_ns && global_ns() - start > q.budget_ns) {
       st |= ST_TIMEOUT;
@@ -606,18 +627,16 @@ __device__ __forceinline__ bool wq_pop(unsigned long long *q, int *count, unsign
   return got;
 }
 
-// Takes the next chunk for the warp. The abort flag lives in host-mapped
-// memory, a round trip over the bus, so a warp polls it (and the time budget)
-// only every 128 chunks it takes.
+// Takes the next chunk for the warp; it asks whether to stop every 128 chunks.
 __device__ __forceinline__ bool take_chunk(unsigned *head, uint32_t n_chunks,
-                                           const uint32_t *abort_flag, unsigned long long budget,
+                                           const StopCtl &stop_ctl, unsigned long long budget,
                                            unsigned long long start, uint32_t &taken,
                                            uint32_t &chunk, uint32_t &st) {
   uint32_t c = 0xFFFFFFFFu;
   if ((threadIdx.x & 31) == 0) {
     bool stop = false;
     if ((taken++ & 127u) == 0u) {
-      if (abort_flag && *((volatile const uint32_t *)abort_flag)) {
+      if (stop_asked(stop_ctl)) {
         st |= ST_ABORTED;
         stop = true;
       } else if (budget && global_ns() - start > budget) {
@@ -644,11 +663,11 @@ constexpr uint32_t CHUNK_RUN = PEN_CHUNK_RUN;
 struct ChunkRun {
   uint32_t next = 0, end = 0;       // chunks [next, end) still to do
   uint32_t unit = 0, unit_end = 0;  // the unit of `next` and the first chunk after it
-  uint32_t taken = 0;               // runs taken (the abort flag is polled every 8)
+  uint32_t taken = 0;               // runs taken (whether to stop is asked every 8)
 };
 
 __device__ __forceinline__ bool next_chunk(ChunkRun &r, const PenState &ps, unsigned *head,
-                                           const uint32_t *abort_flag, unsigned long long budget,
+                                           const StopCtl &stop_ctl, unsigned long long budget,
                                            unsigned long long start, uint32_t &chunk, uint32_t &u,
                                            uint32_t &st) {
   if (r.next >= r.end) {
@@ -656,7 +675,7 @@ __device__ __forceinline__ bool next_chunk(ChunkRun &r, const PenState &ps, unsi
     if ((threadIdx.x & 31) == 0) {
       bool stop = false;
       if ((r.taken++ & 7u) == 0u) {
-        if (abort_flag && *((volatile const uint32_t *)abort_flag)) {
+        if (stop_asked(stop_ctl)) {
           st |= ST_ABORTED;
           stop = true;
         } else if (budget && global_ns() - start > budget) {
@@ -782,7 +801,7 @@ __global__ void k_pen_init(PenState ps) {
 __global__ void __launch_bounds__(256, PEN_INSIDE_MINB) k_pen_inside(const PairView *pairs, const sherd_work_item *items,
                                                     const sherd_candidate *cands, const double *inv,
                                                     PenState ps, unsigned *head,
-                                                    const uint32_t *abort_flag,
+                                                    StopCtl stop_ctl,
                                                     unsigned long long budget, uint32_t *status) {
   __shared__ WarpQueue wqs[8];
   __shared__ unsigned parity[8];
@@ -848,7 +867,7 @@ __global__ void __launch_bounds__(256, PEN_INSIDE_MINB) k_pen_inside(const PairV
   };
   ChunkRun run;
   uint32_t chunk, u;
-  while (next_chunk(run, ps, head, abort_flag, budget, start, chunk, u, st)) {
+  while (next_chunk(run, ps, head, stop_ctl, budget, start, chunk, u, st)) {
     PenUnit x = pen_unit(pairs, items, cands, inv, u);
     uint32_t i = (chunk - ps.chunk0[u]) * 32u + lane;
     bool in_box = false;
@@ -892,7 +911,7 @@ __global__ void k_pen_seed(const PairView *pairs, const sherd_work_item *items,
 __global__ void __launch_bounds__(256) k_pen_min(const PairView *pairs, const sherd_work_item *items,
                                                  const sherd_candidate *cands, const double *inv,
                                                  PenState ps, unsigned *head,
-                                                 const uint32_t *abort_flag,
+                                                 StopCtl stop_ctl,
                                                  unsigned long long budget, uint32_t *status) {
   __shared__ WarpQueue wqs[8];
   WarpQueue &q = wqs[threadIdx.x >> 5];
@@ -914,7 +933,7 @@ __global__ void __launch_bounds__(256) k_pen_min(const PairView *pairs, const sh
     }
   };
   uint32_t chunk, taken = 0;
-  while (take_chunk(head, ps.n_chunks, abort_flag, budget, start, taken, chunk, st)) {
+  while (take_chunk(head, ps.n_chunks, stop_ctl, budget, start, taken, chunk, st)) {
     uint32_t u = unit_of_chunk(ps, chunk);
     PenUnit x = pen_unit(pairs, items, cands, inv, u);
     uint32_t i = (chunk - ps.chunk0[u]) * 32u + lane;

@@ -53,7 +53,11 @@ struct sherd_ctx {
   uint32_t timeout_ms = 0;
   uint32_t *abort_host = nullptr;  // pinned, mapped
   uint32_t *abort_dev = nullptr;
-  uint32_t *d_status = nullptr;
+  uint32_t *d_status = nullptr;  // the status word, and behind it what StopCtl points to
+  static constexpr size_t STATUS_BYTES = 16;
+  StopCtl stop_ctl() const {
+    return {abort_dev, d_status + 1, reinterpret_cast<unsigned long long *>(d_status + 2)};
+  }
   std::map<std::string, MethodStats> stats;
   // Two more streams and their events, to run the ladder's point-count buckets
   // side by side inside the captured ladder graph.
@@ -250,7 +254,7 @@ int finish(sherd_ctx *ctx, const char *method, size_t items, bool timed) {
 
 int begin(sherd_ctx *ctx) {
   CK(cudaSetDevice(ctx->device));
-  CK(cudaMemsetAsync(ctx->d_status, 0, 4, ctx->stream));
+  CK(cudaMemsetAsync(ctx->d_status, 0, sherd_ctx::STATUS_BYTES, ctx->stream));
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   return SHERD_OK;
 }
@@ -753,7 +757,7 @@ int sherd_open(int device, sherd_ctx **out) {
   if ((e = cudaHostAlloc(&ctx->abort_host, 4, cudaHostAllocMapped)) != cudaSuccess) return bad(e);
   *ctx->abort_host = 0;
   if ((e = cudaHostGetDevicePointer(&ctx->abort_dev, ctx->abort_host, 0)) != cudaSuccess) return bad(e);
-  if ((e = cudaMalloc(&ctx->d_status, 4)) != cudaSuccess) return bad(e);
+  if ((e = cudaMalloc(&ctx->d_status, sherd_ctx::STATUS_BYTES)) != cudaSuccess) return bad(e);
   *out = ctx;
   return SHERD_OK;
 }
@@ -1515,7 +1519,7 @@ int sherd_verify(sherd_ctx *ctx, const sherd_surfaces *a, const sherd_surfaces *
       (rc = upload(ctx, order, &zero, 1)) || (rc = upload(ctx, head, &zero, 1)))
     return rc;
   CK(scratch.alloc(v.scratch_floats));
-  QueueCtl q{head.p, order.p, 1, nullptr, 0};
+  QueueCtl q{head.p, order.p, 1, StopCtl{}, 0};
   sherd_params p;
   sherd_params_default(&p);
   k_verify_items<<<1, VER_BLOCK, 0, ctx->stream>>>(dv.p, di.p, q, p, scratch.p, v.scratch_floats, dc.p,
@@ -1693,17 +1697,17 @@ int ladder_stage(sherd_batch *b, cudaStream_t s, unsigned *heads, const uint32_t
   sherd_ctx *ctx = b->ctx;
   unsigned long long budget = (unsigned long long)ctx->timeout_ms * 1000000ULL;
   const bool early = b->early();
-  QueueCtl q0{heads, order, n, ctx->abort_dev, budget};
+  QueueCtl q0{heads, order, n, ctx->stop_ctl(), budget};
   const int wide = b->wide_of(n);
   CK(b->ladder(grid, q0, s, 0, early ? 2 : 4, 0, LADDER_DEFAULT, 0, wide));
   if (early) {
-    QueueCtl q1{heads + 2, order, n, ctx->abort_dev, budget};
+    QueueCtl q1{heads + 2, order, n, ctx->stop_ctl(), budget};
     k_verify_items<<<std::min<unsigned>(b->grid_v, n), VER_BLOCK, 0, s>>>(
         b->dv.p, b->di.p, q1, b->params, b->scratch.p, b->max_scratch, b->dc.p, 0, nullptr, 1, 0,
         ctx->d_status);
     k_early_mark<<<blocks_for(n), 256, 0, s>>>(b->dc.p, order, n, b->params.early_reject_tight);
     CK(cudaGetLastError());
-    QueueCtl q2{heads + 3, order, n, ctx->abort_dev, budget};
+    QueueCtl q2{heads + 3, order, n, ctx->stop_ctl(), budget};
     CK(b->ladder(grid, q2, s, 2, 4, 1, LADDER_DEFAULT, 0, wide));
   }
   return SHERD_OK;
@@ -1727,7 +1731,7 @@ int launch_ladder(sherd_batch *b, cudaStream_t s) {
   for (int bk = 0; bk < sherd_batch::BUCKETS; ++bk) {
     if (!b->seg_count[bk]) continue;
     cudaStream_t on = bk == 0 ? s : ctx->side[bk - 1];
-    QueueCtl q{b->lheads.p + bk, b->dorder.p + b->seg_first[bk], b->seg_count[bk], ctx->abort_dev,
+    QueueCtl q{b->lheads.p + bk, b->dorder.p + b->seg_first[bk], b->seg_count[bk], ctx->stop_ctl(),
                budget};
     CK(b->ladder(b->bucket_grid(bk), q, on, 0, 4, 0, b->variant[bk], b->slot0[bk], b->wide[bk]));
   }
@@ -1753,6 +1757,7 @@ int tune_ladder(sherd_batch *b) {
   cudaStream_t s = ctx->stream;
   int max_occ = 1;
   for (int v = 0; v < LADDER_VARIANTS; ++v) max_occ = std::max(max_occ, b->occ[v]);
+  CK(cudaMemsetAsync(ctx->d_status, 0, sherd_ctx::STATUS_BYTES, s));
   for (int bk = 0; bk < sherd_batch::BUCKETS; ++bk) {
     if (ctx->ladder_tuned[bk] >= 0) {
       b->variant[bk] = ctx->ladder_tuned[bk];
@@ -1766,7 +1771,7 @@ int tune_ladder(sherd_batch *b) {
       const int v = t < 0 ? -1 : t % LADDER_VARIANTS;
       const int run = v < 0 ? LADDER_DEFAULT : v;
       const unsigned grid = std::min<unsigned>(unsigned(b->occ[run] * ctx->sm_count), need);
-      QueueCtl q{b->lheads.p + bk, b->dorder.p + b->seg_first[bk], need, ctx->abort_dev, 0ull};
+      QueueCtl q{b->lheads.p + bk, b->dorder.p + b->seg_first[bk], need, ctx->stop_ctl(), 0ull};
       CK(cudaMemsetAsync(b->lheads.p + bk, 0, sizeof(unsigned), s));
       CK(cudaEventRecord(ctx->ev0, s));
       CK(b->ladder(grid, q, s, 0, 4, 0, run, b->slot0[bk], 0));
@@ -1793,7 +1798,7 @@ int tune_ladder(sherd_batch *b) {
 int launch_verify_items(sherd_batch *b, cudaStream_t s) {
   sherd_ctx *ctx = b->ctx;
   unsigned long long budget = (unsigned long long)ctx->timeout_ms * 1000000ULL;
-  QueueCtl qv{b->heads.p + 1, b->dorder.p, b->n_items, ctx->abort_dev, budget};
+  QueueCtl qv{b->heads.p + 1, b->dorder.p, b->n_items, ctx->stop_ctl(), budget};
   k_verify_items<<<std::min<unsigned>(b->grid_v, b->n_items), VER_BLOCK, 0, s>>>(
       b->dv.p, b->di.p, qv, b->params, b->scratch.p, b->max_scratch, b->dc.p, 1, b->inv.p, 3,
       b->early() ? 1 : 0, ctx->d_status);
@@ -1815,7 +1820,7 @@ int launch_pen_inside(sherd_batch *b, cudaStream_t s) {
   CK(cudaGetLastError());
   if (b->n_chunks) {
     k_pen_inside<<<b->grid_p, 256, 0, s>>>(b->dv.p, b->di.p, b->dc.p, b->inv.p, ps, b->pen_heads.p,
-                                         ctx->abort_dev, budget, ctx->d_status);
+                                         ctx->stop_ctl(), budget, ctx->d_status);
     CK(cudaGetLastError());
   }
   return SHERD_OK;
@@ -1830,7 +1835,7 @@ int launch_pen_min(sherd_batch *b, cudaStream_t s) {
                                                                   b->inv.p, ps, ctx->d_status);
     CK(cudaGetLastError());
     k_pen_min<<<b->grid_m, 256, 0, s>>>(b->dv.p, b->di.p, b->dc.p, b->inv.p, ps,
-                                      b->pen_heads.p + 1, ctx->abort_dev, budget, ctx->d_status);
+                                      b->pen_heads.p + 1, ctx->stop_ctl(), budget, ctx->d_status);
     CK(cudaGetLastError());
   }
   return SHERD_OK;
@@ -2051,7 +2056,7 @@ int batch_run(sherd_batch *b, float *ms) {
       unsigned *heads = b->heads.p + sherd_batch::HEADS * size_t(i);
       const uint32_t *order = b->dorder.p + b->pair_first[i];
       if ((rc = ladder_stage(b, s, heads, order, cnt, cnt))) return rc;
-      QueueCtl qv{heads + 1, order, cnt, ctx->abort_dev, budget};
+      QueueCtl qv{heads + 1, order, cnt, ctx->stop_ctl(), budget};
       k_verify_items<<<std::min<unsigned>(cnt, b->grid_v), VER_BLOCK, 0, s>>>(
           b->dv.p, b->di.p, qv, b->params, b->scratch.p, b->max_scratch, b->dc.p, 1, nullptr, 3,
           b->early() ? 1 : 0, ctx->d_status);
