@@ -885,29 +885,217 @@ __global__ void __launch_bounds__(256, PEN_INSIDE_MINB) k_pen_inside(const PairV
   if (st) atomicOr(status, st);
 }
 
-// The nothing-inside case (verify.rs:569-579): 32 points spread over each such
-// unit seed its shrinking window with unbounded queries.
-__global__ void k_pen_seed(const PairView *pairs, const sherd_work_item *items,
-                           const sherd_candidate *cands, const double *inv, PenState ps,
-                           uint32_t *status) {
-  uint32_t st = 0;
-  uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t u = warp; u < ps.n_units; u += warps) {
-    PenUnit x = pen_unit(pairs, items, cands, inv, u);
-    if (!x.avail || x.n == 0 || ps.deep[u] != 0) continue;
-    if (lane < x.n) {
-      uint32_t i = uint32_t((unsigned long long)lane * x.n / 32u);
-      float window = key2f(*((volatile unsigned *)&ps.best[u]));
-      float d = mesh_distance(*x.mesh, unit_point(x, i), window, st);
-      if (d != f_inf()) atomicMin(&ps.best[u], f2key(d));
+// ---- the minimum distance of the nothing-inside units (verify.rs:569-579) ----
+//
+// A closest-face walk takes 20 nodes on average and thousands at worst, so a
+// warp that walks 32 queries at once waits for the longest of them: 15 times the
+// mean. Here every lane holds a walk of its own and takes one node a round; when
+// enough lanes have finished theirs, the warp refills them from its queue. A
+// walk's bound is the smallest distance its unit has so far, read again as it
+// goes (the unit is only asked for its minimum), so an early answer ends the
+// walks beside it. The result is the smallest of the points' distances whatever
+// the order. For the same reason a walk can be split: with the queue empty, a lane
+// without work takes over the oldest subtree another lane has stacked (the walks
+// of a point thousands of nodes from its answer would otherwise end the kernel
+// alone, 2 us a node).
+
+// Lanes that may be idle before a warp refills them.
+#ifndef MIN_REFILL
+#define MIN_REFILL 4
+#endif
+// Rounds between two looks at what the other walks of the unit have found.
+#ifndef MIN_LOOK
+#define MIN_LOOK 8
+#endif
+
+struct MinWalk {
+  const MeshView *m;
+  unsigned *best;  // f2key of the unit's smallest distance so far
+  F3 p;
+  unsigned key;    // what it was when last looked at
+  float bound2;    // the padded square of it that boxes are held against
+  int node, sb, sp;  // the node to visit, the stack's entries [sb, sp)
+  uint32_t visits;
+};
+
+__device__ __forceinline__ void min_bound(MinWalk &w, unsigned key) {
+  w.key = key;
+  const float b = key2f(key);
+  const float s = b + 4e-6f * b + w.m->pad;
+  w.bound2 = s * s;
+}
+__device__ __forceinline__ void min_look(MinWalk &w) {
+  min_bound(w, *((volatile unsigned *)w.best));
+}
+
+__device__ __forceinline__ void min_leaf(MinWalk &w, int first, int count) {
+  float d = f_inf();
+  for (int s = first; s < first + count; ++s) {
+    F3 a, b, c;
+    uint32_t id;
+    tri_at(*w.m, s, a, b, c, id);
+    d = fminf(d, tri_distance(w.p, a, b, c));
+  }
+  const unsigned key = f2key(d);
+  if (d < f_inf() && key < w.key) {
+    atomicMin(w.best, key);
+    min_bound(w, key);
+  }
+}
+
+// One node of the walk; false when it has ended. mesh_walk with its state kept
+// by the caller.
+__device__ __forceinline__ bool min_step(MinWalk &w, int *stack_n, float *stack_k, uint32_t &st) {
+  if (++w.visits > 2u * w.m->nf + 64u) {
+    st |= ST_STACK;
+    return false;
+  }
+  const Child2 n = load_node(w.m->nodes, w.node);
+  const float pc[3] = {w.p.x, w.p.y, w.p.z};
+  const float k[2] = {box_dist2(n.lo0, n.hi0, pc), box_dist2(n.lo1, n.hi1, pc)};
+  const int near_c = k[1] < k[0] ? 1 : 0;
+  int next = -1;
+  for (int q = 0; q < 2; ++q) {
+    const int c = q == 0 ? near_c : 1 - near_c;
+    if (!(k[c] <= w.bound2)) continue;
+    if (n.cnt[c]) {
+      min_leaf(w, n.ref[c], n.cnt[c]);
+    } else if (next < 0) {
+      next = n.ref[c];
+    } else if (w.sp < STACK) {
+      stack_n[w.sp] = n.ref[c];
+      stack_k[w.sp++] = k[c];
+    } else {
+      st |= ST_STACK;
     }
   }
+  if ((w.visits & (MIN_LOOK - 1)) == 0) min_look(w);
+  if (next < 0) {
+    while (w.sp > w.sb) {
+      --w.sp;
+      if (stack_k[w.sp] <= w.bound2) {
+        next = stack_n[w.sp];
+        break;
+      }
+    }
+  }
+  w.node = next;
+  return next >= 0;
+}
+
+// Starts the walk of point i of unit u; false when there is nothing to walk.
+__device__ __forceinline__ bool min_start(MinWalk &w, const PairView *pairs,
+                                          const sherd_work_item *items, const sherd_candidate *cands,
+                                          const double *inv, const PenState &ps, uint32_t u,
+                                          uint32_t i) {
+  const PenUnit x = pen_unit(pairs, items, cands, inv, u);
+  w.m = x.mesh;
+  w.best = &ps.best[u];
+  w.p = unit_point(x, i);
+  w.node = w.sb = w.sp = 0;
+  w.visits = 0;
+  min_look(w);
+  if (w.m->root_leaf) {
+    min_leaf(w, 0, int(w.m->root_leaf));
+    return false;
+  }
+  return w.m->nf != 0;
+}
+
+// The walks of a warp: `refill(have)` tops the queue up when fewer than 32 of
+// its entries are left (false once there is nothing more to queue).
+template <class Refill>
+__device__ __forceinline__ void min_walks(const PairView *pairs, const sherd_work_item *items,
+                                          const sherd_candidate *cands, const double *inv,
+                                          const PenState &ps, WarpQueue &q, Refill &&refill,
+                                          uint32_t &st) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  int stack_n[STACK];
+  float stack_k[STACK];
+  MinWalk w = {};
+  bool active = false, more = true;
+  for (;;) {
+    const unsigned idle = __ballot_sync(FULL, !active);
+    if (__popc(idle) >= MIN_REFILL) {
+      while (more && q.n_box < 32) more = refill();
+      const int have = q.n_box, rank = __popc(idle & ((1u << lane) - 1u));
+      __syncwarp();
+      if (!active && rank < have) {
+        const unsigned long long e = q.box[have - 1 - rank];
+        active = min_start(w, pairs, items, cands, inv, ps, uint32_t(e >> 32), uint32_t(e));
+      }
+      __syncwarp();
+      if (lane == 0) q.n_box = have - min(have, __popc(idle));
+      __syncwarp();
+      if (have < __popc(idle)) {
+        // The queue is empty: lanes without work take over stacked subtrees.
+        const unsigned poor = __ballot_sync(FULL, !active),
+                       rich = __ballot_sync(FULL, active && w.sp > w.sb);
+        const unsigned below = (1u << lane) - 1u;
+        const int pairs_n = min(__popc(poor), __popc(rich));
+        const bool give = active && w.sp > w.sb && __popc(rich & below) < pairs_n;
+        const bool get = !active && __popc(poor & below) < pairs_n;
+        const int from = get ? int(__fns(rich, 0, __popc(poor & below) + 1)) : lane;
+        int gn = 0;
+        float gk = 0.0f;
+        if (give) {
+          gn = stack_n[w.sb];
+          gk = stack_k[w.sb++];
+        }
+        const int node = __shfl_sync(FULL, gn, from);
+        const float key_k = __shfl_sync(FULL, gk, from);
+        const unsigned long long m = __shfl_sync(FULL, reinterpret_cast<unsigned long long>(w.m), from),
+                                 best = __shfl_sync(FULL, reinterpret_cast<unsigned long long>(w.best), from);
+        const F3 p = {__shfl_sync(FULL, w.p.x, from), __shfl_sync(FULL, w.p.y, from),
+                      __shfl_sync(FULL, w.p.z, from)};
+        const unsigned key = __shfl_sync(FULL, w.key, from), visits = __shfl_sync(FULL, w.visits, from);
+        if (get) {
+          w.m = reinterpret_cast<const MeshView *>(m);
+          w.best = reinterpret_cast<unsigned *>(best);
+          w.p = p;
+          w.node = node;
+          w.sb = w.sp = 0;
+          w.visits = visits;
+          min_bound(w, key);
+          active = key_k <= w.bound2;
+        }
+      }
+      if (!__any_sync(FULL, active) && q.n_box == 0 && !more) return;
+    }
+    if (active) active = min_step(w, stack_n, stack_k, st);
+  }
+}
+
+// 32 points spread over each nothing-inside unit give it a first bound; with
+// none yet, the bound is what the walks beside a walk have found.
+__global__ void __launch_bounds__(256) k_pen_seed(const PairView *pairs, const sherd_work_item *items,
+                                                  const sherd_candidate *cands, const double *inv,
+                                                  PenState ps, uint32_t *status) {
+  __shared__ WarpQueue wqs[8];
+  WarpQueue &q = wqs[threadIdx.x >> 5];
+  const uint32_t lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+  uint32_t st = 0, u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (lane == 0) q.n_box = q.n_in = 0;
+  __syncwarp();
+  min_walks(
+      pairs, items, cands, inv, ps, q,
+      [&]() {
+        if (u >= ps.n_units) return false;
+        const PenUnit x = pen_unit(pairs, items, cands, inv, u);
+        const bool want = x.avail && ps.deep[u] == 0 && lane < x.n;
+        const uint32_t i = uint32_t((unsigned long long)lane * x.n / 32u);
+        wq_push(q.box, &q.n_box, want, (unsigned long long)u << 32 | i);
+        u += warps;
+        return true;
+      },
+      st);
   if (st) atomicOr(status, st);
 }
 
-// The shrinking-window scan over every point of the nothing-inside units; a
-// point farther from the mesh's box than the window cannot beat it.
+// Every point of the nothing-inside units; one farther from the mesh's box than
+// the unit's bound, or out of reach by the bound grid, cannot lower it (the bound
+// only shrinks, so it still cannot when its walk would start).
 __global__ void __launch_bounds__(256) k_pen_min(const PairView *pairs, const sherd_work_item *items,
                                                  const sherd_candidate *cands, const double *inv,
                                                  PenState ps, unsigned *head,
@@ -915,42 +1103,31 @@ __global__ void __launch_bounds__(256) k_pen_min(const PairView *pairs, const sh
                                                  unsigned long long budget, uint32_t *status) {
   __shared__ WarpQueue wqs[8];
   WarpQueue &q = wqs[threadIdx.x >> 5];
-  int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
   if (lane == 0) q.n_box = q.n_in = 0;
   __syncwarp();
-  uint32_t st = 0;
-  unsigned long long start = global_ns();
-  auto query_stage = [&](bool drain) {
-    while (q.n_box >= 32 || (drain && q.n_box > 0)) {
-      unsigned long long e;
-      if (wq_pop(q.box, &q.n_box, e)) {
-        uint32_t u = uint32_t(e >> 32), i = uint32_t(e);
-        PenUnit x = pen_unit(pairs, items, cands, inv, u);
-        float window = key2f(*((volatile unsigned *)&ps.best[u]));
-        float d = mesh_distance(*x.mesh, unit_point(x, i), window, st);
-        if (d != f_inf()) atomicMin(&ps.best[u], f2key(d));
-      }
-    }
-  };
-  uint32_t chunk, taken = 0;
-  while (take_chunk(head, ps.n_chunks, stop_ctl, budget, start, taken, chunk, st)) {
-    uint32_t u = unit_of_chunk(ps, chunk);
-    PenUnit x = pen_unit(pairs, items, cands, inv, u);
-    uint32_t i = (chunk - ps.chunk0[u]) * 32u + lane;
-    bool want = false;
-    if (x.avail && i < x.n && ps.deep[u] == 0) {
-      F3 p = unit_point(x, i);
-      float pc[3] = {p.x, p.y, p.z};
-      float window = key2f(*((volatile unsigned *)&ps.best[u]));
-      float gap = sqrtf(box_dist2(x.mesh->lo, x.mesh->hi, pc));
-      // The window only shrinks, so a point the bound grid puts out of reach
-      // now stays out of reach when its query would run.
-      want = !(gap > window + 1e-5f * window + x.mesh->pad) && mesh_may_reach(*x.mesh, p, window);
-    }
-    wq_push(q.box, &q.n_box, want, (unsigned long long)u << 32 | i);
-    query_stage(false);
-  }
-  query_stage(true);
+  uint32_t st = 0, taken = 0;
+  const unsigned long long start = global_ns();
+  min_walks(
+      pairs, items, cands, inv, ps, q,
+      [&]() {
+        uint32_t chunk;
+        if (!take_chunk(head, ps.n_chunks, stop_ctl, budget, start, taken, chunk, st)) return false;
+        const uint32_t u = unit_of_chunk(ps, chunk);
+        const PenUnit x = pen_unit(pairs, items, cands, inv, u);
+        const uint32_t i = (chunk - ps.chunk0[u]) * 32u + lane;
+        bool want = false;
+        if (x.avail && i < x.n && ps.deep[u] == 0) {
+          const F3 p = unit_point(x, i);
+          const float pc[3] = {p.x, p.y, p.z};
+          const float window = key2f(*((volatile unsigned *)&ps.best[u]));
+          const float gap = sqrtf(box_dist2(x.mesh->lo, x.mesh->hi, pc));
+          want = !(gap > window + 1e-5f * window + x.mesh->pad) && mesh_may_reach(*x.mesh, p, window);
+        }
+        wq_push(q.box, &q.n_box, want, (unsigned long long)u << 32 | i);
+        return true;
+      },
+      st);
   if (st) atomicOr(status, st);
 }
 
