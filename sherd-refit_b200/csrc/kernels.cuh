@@ -561,6 +561,7 @@ struct PenState {
   const uint32_t *chunk0;  // per unit: its first chunk in the flat list (n_units + 1)
   const uint32_t *coarse;  // the unit of every 256th chunk (chunk k << 8)
   uint32_t n_units, n_chunks;
+  uint32_t run;  // chunks per run of the inside pass
 };
 
 struct PenUnit {
@@ -627,38 +628,15 @@ __device__ __forceinline__ bool wq_pop(unsigned long long *q, int *count, unsign
   return got;
 }
 
-// Takes the next chunk for the warp; it asks whether to stop every 128 chunks.
-__device__ __forceinline__ bool take_chunk(unsigned *head, uint32_t n_chunks,
-                                           const StopCtl &stop_ctl, unsigned long long budget,
-                                           unsigned long long start, uint32_t &taken,
-                                           uint32_t &chunk, uint32_t &st) {
-  uint32_t c = 0xFFFFFFFFu;
-  if ((threadIdx.x & 31) == 0) {
-    bool stop = false;
-    if ((taken++ & 127u) == 0u) {
-      if (stop_asked(stop_ctl)) {
-        st |= ST_ABORTED;
-        stop = true;
-      } else if (budget && global_ns() - start > budget) {
-        st |= ST_TIMEOUT;
-        stop = true;
-      }
-    }
-    if (!stop) c = atomicAdd(head, 1u);
-  }
-  chunk = __shfl_sync(0xffffffffu, c, 0);
-  return chunk < n_chunks;
-}
-
-// k_pen_inside takes its chunks in runs: CHUNK_RUN consecutive chunks (of
-// one unit, mostly) per atomic, the unit of each following from the previous
-// one. A unit is then shared by a few dozen warps rather than hundreds, so the
-// running deepest depth its points are checked against is known early, and
-// few points need their depth searched exactly.
-#ifndef PEN_CHUNK_RUN
-#define PEN_CHUNK_RUN 64
-#endif
-constexpr uint32_t CHUNK_RUN = PEN_CHUNK_RUN;
+// k_pen_inside takes its chunks in runs: so many consecutive chunks (of one unit,
+// mostly) per atomic, the unit of each following from the previous one. A unit is
+// then shared by a few dozen warps rather than hundreds, so the running deepest
+// depth its points are checked against is known early, and few points need their
+// depth searched exactly (64 chunks measured best on large batches). A batch with
+// fewer chunks than would give every warp RUNS_PER_WARP runs takes shorter ones:
+// one pair's 12 500 chunks in runs of 64 kept 195 warps of 5920 busy (6.6 ms; in
+// runs of one 0.6 ms).
+constexpr uint32_t RUN_INSIDE = 64, RUNS_PER_WARP = 4;
 
 struct ChunkRun {
   uint32_t next = 0, end = 0;       // chunks [next, end) still to do
@@ -683,12 +661,12 @@ __device__ __forceinline__ bool next_chunk(ChunkRun &r, const PenState &ps, unsi
           stop = true;
         }
       }
-      if (!stop) c = atomicAdd(head, CHUNK_RUN);
+      if (!stop) c = atomicAdd(head, ps.run);
     }
     c = __shfl_sync(0xffffffffu, c, 0);
     if (c >= ps.n_chunks) return false;
     r.next = c;
-    r.end = min(c + CHUNK_RUN, ps.n_chunks);
+    r.end = min(c + ps.run, ps.n_chunks);
     r.unit = unit_of_chunk(ps, c);
     r.unit_end = __ldg(ps.chunk0 + r.unit + 1);
   }
@@ -1095,11 +1073,14 @@ __global__ void __launch_bounds__(256) k_pen_seed(const PairView *pairs, const s
 
 // Every point of the nothing-inside units; one farther from the mesh's box than
 // the unit's bound, or out of reach by the bound grid, cannot lower it (the bound
-// only shrinks, so it still cannot when its walk would start).
+// only shrinks, so it still cannot when its walk would start). The warps stride
+// over the chunks, so that at any time they are all on a few units and each
+// finds the bound the others have brought down: in runs of 8 or 16 chunks a warp,
+// with many units under way at once and their bounds still wide, the pass took
+// 4 to 5 times as long (177 and 230 ms against 44 on a two-wall collection).
 __global__ void __launch_bounds__(256) k_pen_min(const PairView *pairs, const sherd_work_item *items,
                                                  const sherd_candidate *cands, const double *inv,
-                                                 PenState ps, unsigned *head,
-                                                 StopCtl stop_ctl,
+                                                 PenState ps, StopCtl stop_ctl,
                                                  unsigned long long budget, uint32_t *status) {
   __shared__ WarpQueue wqs[8];
   WarpQueue &q = wqs[threadIdx.x >> 5];
@@ -1108,16 +1089,27 @@ __global__ void __launch_bounds__(256) k_pen_min(const PairView *pairs, const sh
   __syncwarp();
   uint32_t st = 0, taken = 0;
   const unsigned long long start = global_ns();
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  uint32_t chunk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   min_walks(
       pairs, items, cands, inv, ps, q,
       [&]() {
-        uint32_t chunk;
-        if (!take_chunk(head, ps.n_chunks, stop_ctl, budget, start, taken, chunk, st)) return false;
-        const uint32_t u = unit_of_chunk(ps, chunk);
+        if (chunk >= ps.n_chunks) return false;
+        if ((taken++ & 127u) == 0u) {
+          if (lane == 0) {
+            if (stop_asked(stop_ctl))
+              st |= ST_ABORTED;
+            else if (budget && global_ns() - start > budget)
+              st |= ST_TIMEOUT;
+          }
+          if (__shfl_sync(0xffffffffu, st & (ST_ABORTED | ST_TIMEOUT), 0)) return false;
+        }
+        const uint32_t u = unit_of_chunk(ps, chunk), i = (chunk - ps.chunk0[u]) * 32u + lane;
+        chunk += warps;
+        if (ps.deep[u] != 0) return true;
         const PenUnit x = pen_unit(pairs, items, cands, inv, u);
-        const uint32_t i = (chunk - ps.chunk0[u]) * 32u + lane;
         bool want = false;
-        if (x.avail && i < x.n && ps.deep[u] == 0) {
+        if (x.avail && i < x.n) {
           const F3 p = unit_point(x, i);
           const float pc[3] = {p.x, p.y, p.z};
           const float window = key2f(*((volatile unsigned *)&ps.best[u]));

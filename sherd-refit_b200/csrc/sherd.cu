@@ -1807,15 +1807,16 @@ int launch_verify_items(sherd_batch *b, cudaStream_t s) {
 }
 
 PenState pen_state(sherd_batch *b) {
+  const uint32_t run = std::max(1u, std::min(RUN_INSIDE, b->n_chunks / (b->grid_p * 8u * RUNS_PER_WARP)));
   return PenState{b->deeper.p, b->deep.p, b->best.p, b->chunk0.p, b->coarse.p, 2 * b->n_items,
-                  b->n_chunks};
+                  b->n_chunks, run};
 }
 
 int launch_pen_inside(sherd_batch *b, cudaStream_t s) {
   sherd_ctx *ctx = b->ctx;
   unsigned long long budget = (unsigned long long)ctx->timeout_ms * 1000000ULL;
   PenState ps = pen_state(b);
-  CK(cudaMemsetAsync(b->pen_heads.p, 0, 2 * sizeof(unsigned), s));
+  CK(cudaMemsetAsync(b->pen_heads.p, 0, sizeof(unsigned), s));
   k_pen_init<<<blocks_for(ps.n_units), 256, 0, s>>>(ps);
   CK(cudaGetLastError());
   if (b->n_chunks) {
@@ -1835,7 +1836,7 @@ int launch_pen_min(sherd_batch *b, cudaStream_t s) {
                                                                   b->inv.p, ps, ctx->d_status);
     CK(cudaGetLastError());
     k_pen_min<<<b->grid_m, 256, 0, s>>>(b->dv.p, b->di.p, b->dc.p, b->inv.p, ps,
-                                      b->pen_heads.p + 1, ctx->stop_ctl(), budget, ctx->d_status);
+                                      ctx->stop_ctl(), budget, ctx->d_status);
     CK(cudaGetLastError());
   }
   return SHERD_OK;
@@ -1988,7 +1989,7 @@ int batch_create(sherd_ctx *ctx, sherd_pair *const *pairs, uint32_t n_pairs,
     CK(b->deeper.alloc(2 * size_t(n_items)));
     CK(b->deep.alloc(2 * size_t(n_items)));
     CK(b->best.alloc(2 * size_t(n_items)));
-    CK(b->pen_heads.alloc(2));
+    CK(b->pen_heads.alloc(1));
     int occ_p = 0, occ_m = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_p, k_pen_inside, 256, 0));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_m, k_pen_min, 256, 0));
