@@ -906,14 +906,48 @@ __device__ __forceinline__ void min_look(MinWalk &w) {
   min_bound(w, *((volatile unsigned *)w.best));
 }
 
-__device__ __forceinline__ void min_leaf(MinWalk &w, int first, int count) {
-  float d = f_inf();
-  for (int s = first; s < first + count; ++s) {
-    F3 a, b, c;
-    uint32_t id;
-    tri_at(*w.m, s, a, b, c, id);
-    d = fminf(d, tri_distance(w.p, a, b, c));
+// The faces of the leaves the warp's walks have come to, shared out over its
+// lanes: leaf `count` faces at `first` of each lane (0: none), laid end to end.
+// A lane's own loop over its faces has the others wait for up to twelve
+// face tests, a load and a division each; 32 at a time they take about three
+// rounds. Returns the smallest distance of the lane's faces to its point.
+__device__ __forceinline__ float warp_leaves(const MeshView *m, F3 p, uint32_t first, uint32_t count,
+                                             unsigned *slot) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  uint32_t incl = count;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += y;
   }
+  const uint32_t off = incl - count, total = __shfl_sync(FULL, incl, 31);
+  if (!total) return f_inf();
+  slot[lane] = f2key(f_inf());
+  __syncwarp();
+  const unsigned long long tri = reinterpret_cast<unsigned long long>(count ? m->tri : nullptr);
+  for (uint32_t base = 0; base < total; base += 32) {
+    const uint32_t w = base + lane;
+    int j = 0;  // the last lane whose faces start at or before w
+#pragma unroll
+    for (int step = 16; step; step >>= 1)
+      if (__shfl_sync(FULL, off, j + step) <= w) j += step;
+    const F3 q = {__shfl_sync(FULL, p.x, j), __shfl_sync(FULL, p.y, j), __shfl_sync(FULL, p.z, j)};
+    const uint32_t fj = __shfl_sync(FULL, first, j), oj = __shfl_sync(FULL, off, j);
+    const float4 *t = reinterpret_cast<const float4 *>(__shfl_sync(FULL, tri, j)) + 3 * size_t(fj + (w - oj));
+    if (w < total) {
+      const float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t + 2);
+      const float d = tri_distance(q, {a.x, a.y, a.z}, {b.x, b.y, b.z}, {c.x, c.y, c.z});
+      if (d < f_inf()) atomicMin(&slot[j], f2key(d));
+    }
+  }
+  __syncwarp();
+  const float d = key2f(slot[lane]);
+  __syncwarp();
+  return d;
+}
+
+__device__ __forceinline__ void min_found(MinWalk &w, float d) {
   const unsigned key = f2key(d);
   if (d < f_inf() && key < w.key) {
     atomicMin(w.best, key);
@@ -921,32 +955,50 @@ __device__ __forceinline__ void min_leaf(MinWalk &w, int first, int count) {
   }
 }
 
-// One node of the walk; false when it has ended. mesh_walk with its state kept
-// by the caller.
-__device__ __forceinline__ bool min_step(MinWalk &w, int *stack_n, float *stack_k, uint32_t &st) {
-  if (++w.visits > 2u * w.m->nf + 64u) {
+// One node of every lane's walk (`active`: it has one); false where it has ended.
+// mesh_walk with its state kept by the caller and the leaves shared out.
+__device__ __forceinline__ bool min_step(MinWalk &w, bool active, int *stack_n, float *stack_k,
+                                         unsigned *slot, uint32_t &st) {
+  if (active && ++w.visits > 2u * w.m->nf + 64u) {
     st |= ST_STACK;
-    return false;
+    active = false;
   }
-  const Child2 n = load_node(w.m->nodes, w.node);
-  const float pc[3] = {w.p.x, w.p.y, w.p.z};
-  const float k[2] = {box_dist2(n.lo0, n.hi0, pc), box_dist2(n.lo1, n.hi1, pc)};
-  const int near_c = k[1] < k[0] ? 1 : 0;
-  int next = -1;
-  for (int q = 0; q < 2; ++q) {
-    const int c = q == 0 ? near_c : 1 - near_c;
-    if (!(k[c] <= w.bound2)) continue;
-    if (n.cnt[c]) {
-      min_leaf(w, n.ref[c], n.cnt[c]);
-    } else if (next < 0) {
-      next = n.ref[c];
-    } else if (w.sp < STACK) {
-      stack_n[w.sp] = n.ref[c];
-      stack_k[w.sp++] = k[c];
-    } else {
-      st |= ST_STACK;
+  int next = -1, leaf[2] = {0, 0};
+  uint32_t faces[2] = {0, 0};
+  if (active) {
+    const Child2 n = load_node(w.m->nodes, w.node);
+    const float pc[3] = {w.p.x, w.p.y, w.p.z};
+    const float k[2] = {box_dist2(n.lo0, n.hi0, pc), box_dist2(n.lo1, n.hi1, pc)};
+    const bool in0 = k[0] <= w.bound2, in1 = k[1] <= w.bound2;
+    if (in0 && n.cnt[0]) {
+      leaf[0] = n.ref[0];
+      faces[0] = n.cnt[0];
+    }
+    if (in1 && n.cnt[1]) {
+      leaf[1] = n.ref[1];
+      faces[1] = n.cnt[1];
+    }
+    const bool go0 = in0 && !n.cnt[0], go1 = in1 && !n.cnt[1];
+    if (go0 && go1) {
+      const bool second = k[1] < k[0];
+      next = second ? n.ref[1] : n.ref[0];
+      if (w.sp < STACK) {
+        stack_n[w.sp] = second ? n.ref[0] : n.ref[1];
+        stack_k[w.sp++] = second ? k[0] : k[1];
+      } else {
+        st |= ST_STACK;
+      }
+    } else if (go0 || go1) {
+      next = go0 ? n.ref[0] : n.ref[1];
     }
   }
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    if (!__any_sync(0xffffffffu, faces[c] != 0)) continue;
+    const float d = warp_leaves(w.m, w.p, leaf[c], faces[c], slot);
+    if (faces[c]) min_found(w, d);
+  }
+  if (!active) return false;
   if ((w.visits & (MIN_LOOK - 1)) == 0) min_look(w);
   if (next < 0) {
     while (w.sp > w.sb) {
@@ -974,7 +1026,12 @@ __device__ __forceinline__ bool min_start(MinWalk &w, const PairView *pairs,
   w.visits = 0;
   min_look(w);
   if (w.m->root_leaf) {
-    min_leaf(w, 0, int(w.m->root_leaf));
+    for (uint32_t f = 0; f < w.m->root_leaf; ++f) {
+      F3 a, b, c;
+      uint32_t id;
+      tri_at(*w.m, f, a, b, c, id);
+      min_found(w, tri_distance(w.p, a, b, c));
+    }
     return false;
   }
   return w.m->nf != 0;
@@ -985,8 +1042,8 @@ __device__ __forceinline__ bool min_start(MinWalk &w, const PairView *pairs,
 template <class Refill>
 __device__ __forceinline__ void min_walks(const PairView *pairs, const sherd_work_item *items,
                                           const sherd_candidate *cands, const double *inv,
-                                          const PenState &ps, WarpQueue &q, Refill &&refill,
-                                          uint32_t &st) {
+                                          const PenState &ps, WarpQueue &q, unsigned *slot,
+                                          Refill &&refill, uint32_t &st) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   int stack_n[STACK];
@@ -1041,7 +1098,7 @@ __device__ __forceinline__ void min_walks(const PairView *pairs, const sherd_wor
       }
       if (!__any_sync(FULL, active) && q.n_box == 0 && !more) return;
     }
-    if (active) active = min_step(w, stack_n, stack_k, st);
+    active = min_step(w, active, stack_n, stack_k, slot, st);
   }
 }
 
@@ -1051,13 +1108,14 @@ __global__ void __launch_bounds__(256) k_pen_seed(const PairView *pairs, const s
                                                   const sherd_candidate *cands, const double *inv,
                                                   PenState ps, uint32_t *status) {
   __shared__ WarpQueue wqs[8];
+  __shared__ unsigned slots[8][32];
   WarpQueue &q = wqs[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
   uint32_t st = 0, u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (lane == 0) q.n_box = q.n_in = 0;
   __syncwarp();
   min_walks(
-      pairs, items, cands, inv, ps, q,
+      pairs, items, cands, inv, ps, q, slots[threadIdx.x >> 5],
       [&]() {
         if (u >= ps.n_units) return false;
         const PenUnit x = pen_unit(pairs, items, cands, inv, u);
@@ -1083,6 +1141,7 @@ __global__ void __launch_bounds__(256) k_pen_min(const PairView *pairs, const sh
                                                  PenState ps, StopCtl stop_ctl,
                                                  unsigned long long budget, uint32_t *status) {
   __shared__ WarpQueue wqs[8];
+  __shared__ unsigned slots[8][32];
   WarpQueue &q = wqs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   if (lane == 0) q.n_box = q.n_in = 0;
@@ -1092,7 +1151,7 @@ __global__ void __launch_bounds__(256) k_pen_min(const PairView *pairs, const sh
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   uint32_t chunk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   min_walks(
-      pairs, items, cands, inv, ps, q,
+      pairs, items, cands, inv, ps, q, slots[threadIdx.x >> 5],
       [&]() {
         if (chunk >= ps.n_chunks) return false;
         if ((taken++ & 127u) == 0u) {
