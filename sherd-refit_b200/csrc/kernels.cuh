@@ -370,13 +370,14 @@ constexpr int LADDER_DEFAULT = 1;
 // for their first chunk), so one thread at a time reads it, every POLL_NS, and
 // the rest read its copy on the device. The copy is cleared with the status word.
 struct StopCtl {
-  const uint32_t *host;       // host-mapped; non-zero asks the kernel to stop
+  const uint32_t *host;       // host-mapped; non-zero asks the kernel to stop (null: never)
   uint32_t *seen;             // the device's copy
   unsigned long long *polled; // when it was last refreshed (global_ns)
 };
 constexpr unsigned long long POLL_NS = 20000;
 
 __device__ __forceinline__ bool stop_asked(const StopCtl &c) {
+  if (!c.host) return false;
   if (*((volatile uint32_t *)c.seen)) return true;
   const unsigned long long last = *((volatile unsigned long long *)c.polled), now = global_ns();
   if (now - last < POLL_NS || atomicCAS(c.polled, last, now) != last) return false;
@@ -400,7 +401,7 @@ __device__ __forceinline__ bool take(const QueueCtl &q, unsigned long long start
   __shared__ unsigned s_item;
   if (threadIdx.x == 0) {
     unsigned item = 0xFFFFFFFFu;
-    if (q.stop.host && stop_asked(q.stop)) {
+    if (stop_asked(q.stop)) {
       st |= ST_ABORTED;
     } else if (q.budget_ns && global_ns() - start > q.budget_ns) {
       st |= ST_TIMEOUT;
@@ -513,6 +514,87 @@ __global__ void __launch_bounds__(VER_BLOCK, 3) k_verify_items(const PairView *p
                  inv ? inv + 16 * size_t(it) : nullptr);
   }
   if (st) atomicOr(status, st);
+}
+
+// k_verify_items for few items, the penetration left to the wavefront kernels: the
+// four scores of an item (the two fracture sides, the seam, the continuity) on a
+// block each, of 1024 threads, side by side. What an item takes is then its
+// longest score's few rounds of queries, where one 256-thread block went through
+// all four: ten items 1.26 ms, 0.35 ms this way. With more blocks than two per SM
+// the SMs are full either way and the persistent form stays (verify_in_parts).
+constexpr int PART_BLOCK = 1024;
+__global__ void __launch_bounds__(PART_BLOCK) k_verify_parts(const PairView *pairs,
+                                                             const sherd_work_item *items,
+                                                             unsigned *scratch, size_t stride,
+                                                             sherd_candidate *out, int full,
+                                                             double *inv, int pose_rung,
+                                                             uint32_t *status) {
+  __shared__ VerShared sh;
+  uint32_t st = 0;
+  const uint32_t it = blockIdx.x >> 2, part = blockIdx.x & 3u;
+  const PairView &pr = pairs[items[it].pair];
+  sherd_candidate *c = out + it;
+  unsigned *mine = scratch + stride * blockIdx.x;
+  if (threadIdx.x < 16) sh.t[threadIdx.x] = c->rungs[pose_rung].transform[threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x == 0) pose_inverse(sh.t, sh.inv);
+  __syncthreads();
+  const sherd_scales &sc = pr.sc;
+  double x = 0.0, y = 0.0, z = 0.0;
+  if (part == 0) {
+    if (threadIdx.x < 16) inv[16 * size_t(it) + threadIdx.x] = sh.inv[threadIdx.x];
+    one_side(pr.b.pf, pr.b.n_pf, sh.t, pr.a.frac, pr.b.frac_area, sc, mine, sh, x, y, z, st);
+  } else if (part == 1) {
+    one_side(pr.a.pf, pr.a.n_pf, sh.inv, pr.b.frac, pr.a.frac_area, sc, mine, sh, x, y, z, st);
+  } else if (part == 2) {
+    x = seam_score(pr, sh, st);
+  } else {
+    x = 1.0;
+    y = -1.0;
+    if (full) {
+      unsigned long long *steps = reinterpret_cast<unsigned long long *>(mine);
+      continuity(pr, steps, steps + pr.b.n_margin, sh, x, y, st);
+    }
+  }
+  if (threadIdx.x == 0) {
+    sherd_scores &s = c->scores;
+    if (part == 0) {
+      s.tight_b = x;
+      s.gap_b = y;
+      s.contact_b = z;
+    } else if (part == 1) {
+      s.tight_a = x;
+      s.gap_a = y;
+      s.contact_a = z;
+    } else if (part == 2) {
+      s.seam = x;
+    } else {
+      s.cont = x;
+      s.cont_n = y;
+    }
+  }
+  if (st) atomicOr(status, st);
+}
+
+// The rest of an item's scores, as verify_block leaves them.
+__global__ void k_verify_join(const PairView *pairs, const sherd_work_item *items,
+                              sherd_candidate *out, int full, uint32_t n) {
+  const uint32_t it = blockIdx.x * blockDim.x + threadIdx.x;
+  if (it >= n) return;
+  const PairView &pr = pairs[items[it].pair];
+  sherd_scores &s = out[it].scores;
+  s.tight = fmin(s.tight_a, s.tight_b);
+  s.gap = fmax(s.gap_a, s.gap_b);
+  s.contact = fmin(s.contact_a, s.contact_b);
+  s.gap_limit = pr.sc.gap / pr.sc.t;
+  s.tight_delta = pr.sc.tight / pr.sc.t;
+  s.pen = 0.0;
+  s.pen_depth = 0.0;
+  s.pen_unavailable =
+      full && (!pr.a.has_mesh || !pr.b.has_mesh || !(pr.a.watertight && pr.b.watertight)) ? 1u : 0u;
+  s.partial = full ? 0u : 1u;
+  s.brk = 0.0;
+  s.brk_best = 0.0;
 }
 
 // R 5.6's early rejection (pair.rs:315-340) after the fracture and seam

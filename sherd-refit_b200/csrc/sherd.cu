@@ -1494,44 +1494,6 @@ int pair_view(sherd_ctx *ctx, const sherd_surfaces *a, const sherd_surfaces *b, 
 
 }  // namespace
 
-int sherd_verify(sherd_ctx *ctx, const sherd_surfaces *a, const sherd_surfaces *b, const double pose[16],
-                 const sherd_scales *sc, int full, sherd_scores *out) {
-  if (!ctx || !a || !b || !sc || !out) return fail(ctx, SHERD_E_INVALID, "null argument");
-  if (!finite_pose(pose)) return fail(ctx, SHERD_E_INVALID, "pose is not finite");
-  if (!(sc->t > 0.0)) return fail(ctx, SHERD_E_INVALID, "scales need t > 0");
-  CtxLock lock(ctx);
-  int rc = begin(ctx);
-  if (rc) return rc;
-  DBuf<uint32_t> cells;
-  PairView v;
-  if ((rc = pair_view(ctx, a, b, sc, cells, v))) return rc;
-  DBuf<PairView> dv;
-  DBuf<sherd_work_item> di;
-  DBuf<sherd_candidate> dc;
-  DBuf<uint32_t> order;
-  DBuf<unsigned> head, scratch;
-  sherd_work_item item{};
-  std::memcpy(item.init, pose, sizeof item.init);
-  sherd_candidate cand{};
-  std::memcpy(cand.rungs[3].transform, pose, sizeof cand.rungs[3].transform);
-  uint32_t zero = 0;
-  if ((rc = upload(ctx, dv, &v, 1)) || (rc = upload(ctx, di, &item, 1)) || (rc = upload(ctx, dc, &cand, 1)) ||
-      (rc = upload(ctx, order, &zero, 1)) || (rc = upload(ctx, head, &zero, 1)))
-    return rc;
-  CK(scratch.alloc(v.scratch_floats));
-  QueueCtl q{head.p, order.p, 1, StopCtl{}, 0};
-  sherd_params p;
-  sherd_params_default(&p);
-  k_verify_items<<<1, VER_BLOCK, 0, ctx->stream>>>(dv.p, di.p, q, p, scratch.p, v.scratch_floats, dc.p,
-                                                  full, nullptr, 3, 0, ctx->d_status);
-  CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(&cand, dc.p, sizeof cand, cudaMemcpyDeviceToHost, ctx->stream));
-  rc = finish(ctx, "verify", 1, true);
-  if (rc) return rc;
-  *out = cand.scores;
-  return SHERD_OK;
-}
-
 // ---- the batched stage-2 path ---------------------------------------------------
 
 int sherd_pair_create(sherd_ctx *ctx, const sherd_surfaces *a, const sherd_surfaces *b,
@@ -1591,6 +1553,11 @@ int sherd_pair_free(sherd_pair *pair) {
 
 struct sherd_batch {
   sherd_ctx *ctx = nullptr;
+  bool verify_only = false;  // no ladder, and nothing stops it
+  StopCtl stop() const { return verify_only ? StopCtl{} : ctx->stop_ctl(); }
+  unsigned long long budget() const {
+    return verify_only ? 0ull : (unsigned long long)ctx->timeout_ms * 1000000ULL;
+  }
   int sched = SHERD_SCHED_BATCHED;
   uint32_t n_pairs = 0, n_items = 0;
   sherd_params params{};
@@ -1795,16 +1762,32 @@ int tune_ladder(sherd_batch *b) {
   return SHERD_OK;
 }
 
-int launch_verify_items(sherd_batch *b, cudaStream_t s) {
+// Whether n items' scores go side by side (k_verify_parts): while the blocks of
+// their parts leave an SM no more than two.
+bool verify_in_parts(const sherd_batch *b, uint32_t n) {
+  return 4ull * n <= std::min<uint64_t>(2ull * b->ctx->sm_count, b->grid_v);
+}
+
+int launch_verify(sherd_batch *b, cudaStream_t s, int full) {
   sherd_ctx *ctx = b->ctx;
-  unsigned long long budget = (unsigned long long)ctx->timeout_ms * 1000000ULL;
-  QueueCtl qv{b->heads.p + 1, b->dorder.p, b->n_items, ctx->stop_ctl(), budget};
+  if (!b->early() && verify_in_parts(b, b->n_items)) {
+    k_verify_parts<<<4 * b->n_items, PART_BLOCK, 0, s>>>(b->dv.p, b->di.p, b->scratch.p,
+                                                         b->max_scratch, b->dc.p, full, b->inv.p, 3,
+                                                         ctx->d_status);
+    CK(cudaGetLastError());
+    k_verify_join<<<blocks_for(b->n_items), 256, 0, s>>>(b->dv.p, b->di.p, b->dc.p, full, b->n_items);
+    CK(cudaGetLastError());
+    return SHERD_OK;
+  }
+  QueueCtl qv{b->heads.p + 1, b->dorder.p, b->n_items, b->stop(), b->budget()};
   k_verify_items<<<std::min<unsigned>(b->grid_v, b->n_items), VER_BLOCK, 0, s>>>(
-      b->dv.p, b->di.p, qv, b->params, b->scratch.p, b->max_scratch, b->dc.p, 1, b->inv.p, 3,
+      b->dv.p, b->di.p, qv, b->params, b->scratch.p, b->max_scratch, b->dc.p, full, b->inv.p, 3,
       b->early() ? 1 : 0, ctx->d_status);
   CK(cudaGetLastError());
   return SHERD_OK;
 }
+
+int launch_verify_items(sherd_batch *b, cudaStream_t s) { return launch_verify(b, s, 1); }
 
 PenState pen_state(sherd_batch *b) {
   const uint32_t run = std::max(1u, std::min(RUN_INSIDE, b->n_chunks / (b->grid_p * 8u * RUNS_PER_WARP)));
@@ -1814,14 +1797,13 @@ PenState pen_state(sherd_batch *b) {
 
 int launch_pen_inside(sherd_batch *b, cudaStream_t s) {
   sherd_ctx *ctx = b->ctx;
-  unsigned long long budget = (unsigned long long)ctx->timeout_ms * 1000000ULL;
   PenState ps = pen_state(b);
   CK(cudaMemsetAsync(b->pen_heads.p, 0, sizeof(unsigned), s));
   k_pen_init<<<blocks_for(ps.n_units), 256, 0, s>>>(ps);
   CK(cudaGetLastError());
   if (b->n_chunks) {
     k_pen_inside<<<b->grid_p, 256, 0, s>>>(b->dv.p, b->di.p, b->dc.p, b->inv.p, ps, b->pen_heads.p,
-                                         ctx->stop_ctl(), budget, ctx->d_status);
+                                         b->stop(), b->budget(), ctx->d_status);
     CK(cudaGetLastError());
   }
   return SHERD_OK;
@@ -1829,14 +1811,13 @@ int launch_pen_inside(sherd_batch *b, cudaStream_t s) {
 
 int launch_pen_min(sherd_batch *b, cudaStream_t s) {
   sherd_ctx *ctx = b->ctx;
-  unsigned long long budget = (unsigned long long)ctx->timeout_ms * 1000000ULL;
   PenState ps = pen_state(b);
   if (b->n_chunks) {
     k_pen_seed<<<blocks_for(size_t(ps.n_units) * 32), 256, 0, s>>>(b->dv.p, b->di.p, b->dc.p,
                                                                   b->inv.p, ps, ctx->d_status);
     CK(cudaGetLastError());
     k_pen_min<<<b->grid_m, 256, 0, s>>>(b->dv.p, b->di.p, b->dc.p, b->inv.p, ps,
-                                      ctx->stop_ctl(), budget, ctx->d_status);
+                                      b->stop(), b->budget(), ctx->d_status);
     CK(cudaGetLastError());
   }
   return SHERD_OK;
@@ -1874,22 +1855,26 @@ int capture_one(sherd_batch *b, int (*launch)(sherd_batch *, cudaStream_t), cuda
   return SHERD_OK;
 }
 
+int (*const kStages[sherd_batch::STAGES])(sherd_batch *, cudaStream_t) = {
+    launch_ladder, launch_verify_items, launch_pen_inside, launch_pen_min, launch_finalize};
+
 // Captures every stage's graph (again when the time budget changed).
 int capture(sherd_batch *b) {
   if (b->exec[0] && b->captured_timeout == b->ctx->timeout_ms) return SHERD_OK;
-  int (*stage[sherd_batch::STAGES])(sherd_batch *, cudaStream_t) = {
-      launch_ladder, launch_verify_items, launch_pen_inside, launch_pen_min, launch_finalize};
   for (int k = 0; k < sherd_batch::STAGES; ++k) {
-    int rc = capture_one(b, stage[k], b->graph[k], b->exec[k]);
+    int rc = capture_one(b, kStages[k], b->graph[k], b->exec[k]);
     if (rc) return rc;
   }
   b->captured_timeout = b->ctx->timeout_ms;
   return SHERD_OK;
 }
 
-int batch_create(sherd_ctx *ctx, sherd_pair *const *pairs, uint32_t n_pairs,
-                 const sherd_work_item *items, uint32_t n_items, const sherd_params *p, int sched,
-                 sherd_batch *b) {
+// Sizes and uploads a batch; `resident`: its stages are captured as graphs, to be
+// run again and again (a batch run once launches its kernels directly: capturing
+// and instantiating the five graphs takes 0.7 ms).
+int batch_create(sherd_ctx *ctx, const std::vector<PairView> &views, const sherd_work_item *items,
+                 uint32_t n_items, const sherd_params *p, int sched, bool resident, sherd_batch *b) {
+  const uint32_t n_pairs = uint32_t(views.size());
   b->ctx = ctx;
   b->sched = sched;
   b->n_pairs = n_pairs;
@@ -1899,15 +1884,13 @@ int batch_create(sherd_ctx *ctx, sherd_pair *const *pairs, uint32_t n_pairs,
   // of the verification, per pair.
   std::vector<double> pair_cost(n_pairs);
   for (uint32_t i = 0; i < n_pairs; ++i) {
-    const PairView &v = pairs[i]->view;
+    const PairView &v = views[i];
     pair_cost[i] = 60.0 * (double(v.n_reg) + double(v.n_frac)) + 4.0 * (v.a.n_s + v.b.n_s) +
                    double(v.a.n_pf + v.b.n_pf);
     b->max_scratch = std::max(b->max_scratch, v.scratch_floats);
     b->hint_stride = std::max<size_t>(b->hint_stride, std::max(v.n_reg, v.n_frac));
     if (v.reg_tgt.n >= 0xFFFFu || v.frac_tgt.n >= 0xFFFFu) b->hint16 = false;
   }
-  std::vector<PairView> views(n_pairs);
-  for (uint32_t i = 0; i < n_pairs; ++i) views[i] = pairs[i]->view;
   std::vector<uint32_t> order(n_items);
   if (sched == SHERD_SCHED_BATCHED) {
     // By point-count bucket of the moving clouds (> 16384, > 4096, the rest),
@@ -2022,11 +2005,17 @@ int batch_create(sherd_ctx *ctx, sherd_pair *const *pairs, uint32_t n_pairs,
   CK(b->mem.alloc(b->hint_stride, slots, ints ? sizeof(int) : sizeof(uint16_t)));
   for (cudaEvent_t &e : b->ev) CK(cudaEventCreate(&e));
   CK(cudaStreamSynchronize(ctx->stream));
-  if (sched == SHERD_SCHED_BATCHED) {
+  if (sched == SHERD_SCHED_BATCHED && !b->verify_only) {
     if (!b->early() && (rc = tune_ladder(b))) return rc;
-    return capture(b);
+    if (resident) return capture(b);
   }
   return SHERD_OK;
+}
+
+std::vector<PairView> pair_views(sherd_pair *const *pairs, uint32_t n) {
+  std::vector<PairView> v(n);
+  for (uint32_t i = 0; i < n; ++i) v[i] = pairs[i]->view;
+  return v;
 }
 
 int batch_run(sherd_batch *b, float *ms) {
@@ -2040,11 +2029,14 @@ int batch_run(sherd_batch *b, float *ms) {
     static const char *const kStage[sherd_batch::STAGES] = {
         "sherd stage ladder", "sherd stage verify", "sherd stage pen_inside", "sherd stage pen_min",
         "sherd stage finalize"};
-    if ((rc = capture(b))) return rc;
+    if (b->exec[0] && (rc = capture(b))) return rc;
     CK(cudaEventRecord(b->ev[0], s));
     for (int k = 0; k < sherd_batch::STAGES; ++k) {
       NvtxRange stage(kStage[k]);
-      CK(cudaGraphLaunch(b->exec[k], s));
+      if (b->exec[k])
+        CK(cudaGraphLaunch(b->exec[k], s));
+      else if ((rc = kStages[k](b, s)))
+        return rc;
       CK(cudaEventRecord(b->ev[k + 1], s));
     }
   } else {
@@ -2098,6 +2090,41 @@ int check_batch_args(sherd_ctx *ctx, sherd_pair *const *pairs, uint32_t n_pairs,
 
 extern "C" {
 
+// One pose through the batch's own stages past the ladder: the scores in parts, the
+// penetration as a wavefront over the device (a single block took 5 ms for it).
+int sherd_verify(sherd_ctx *ctx, const sherd_surfaces *a, const sherd_surfaces *b, const double pose[16],
+                 const sherd_scales *sc, int full, sherd_scores *out) {
+  if (!ctx || !a || !b || !sc || !out) return fail(ctx, SHERD_E_INVALID, "null argument");
+  if (!finite_pose(pose)) return fail(ctx, SHERD_E_INVALID, "pose is not finite");
+  if (!(sc->t > 0.0)) return fail(ctx, SHERD_E_INVALID, "scales need t > 0");
+  CtxLock lock(ctx);
+  int rc = begin(ctx);
+  if (rc) return rc;
+  DBuf<uint32_t> cells;
+  std::vector<PairView> views(1);
+  if ((rc = pair_view(ctx, a, b, sc, cells, views[0]))) return rc;
+  sherd_work_item item{};
+  std::memcpy(item.init, pose, sizeof item.init);
+  sherd_candidate cand{};
+  std::memcpy(cand.rungs[3].transform, pose, sizeof cand.rungs[3].transform);
+  sherd_params p;
+  sherd_params_default(&p);
+  p.early_reject_tight = 0.0;
+  sherd_batch one;
+  one.verify_only = true;
+  if ((rc = batch_create(ctx, views, &item, 1, &p, SHERD_SCHED_BATCHED, false, &one))) return rc;
+  CK(cudaMemcpyAsync(one.dc.p, &cand, sizeof cand, cudaMemcpyHostToDevice, ctx->stream));
+  if ((rc = launch_verify(&one, ctx->stream, full ? 1 : 0))) return rc;
+  if (full)
+    for (auto stage : {launch_pen_inside, launch_pen_min, launch_finalize})
+      if ((rc = stage(&one, ctx->stream))) return rc;
+  CK(cudaMemcpyAsync(&cand, one.dc.p, sizeof cand, cudaMemcpyDeviceToHost, ctx->stream));
+  rc = finish(ctx, "verify", 1, true);
+  if (rc) return rc;
+  *out = cand.scores;
+  return SHERD_OK;
+}
+
 int sherd_batch_create(sherd_ctx *ctx, sherd_pair *const *pairs, uint32_t n_pairs,
                        const sherd_work_item *items, uint32_t n_items, const sherd_params *p,
                        int sched, sherd_batch **out) {
@@ -2109,7 +2136,7 @@ int sherd_batch_create(sherd_ctx *ctx, sherd_pair *const *pairs, uint32_t n_pair
   CtxLock lock(ctx);
   CK(cudaSetDevice(ctx->device));
   sherd_batch *b = new sherd_batch;
-  rc = batch_create(ctx, pairs, n_pairs, items, n_items, p, sched, b);
+  rc = batch_create(ctx, pair_views(pairs, n_pairs), items, n_items, p, sched, true, b);
   if (rc) {
     delete b;
     return rc;
@@ -2153,7 +2180,7 @@ int sherd_ladder_verify_batch(sherd_ctx *ctx, sherd_pair *const *pairs, uint32_t
   CtxLock lock(ctx);
   CK(cudaSetDevice(ctx->device));
   sherd_batch b;
-  if ((rc = batch_create(ctx, pairs, n_pairs, items, n_items, p, sched, &b))) return rc;
+  if ((rc = batch_create(ctx, pair_views(pairs, n_pairs), items, n_items, p, sched, false, &b))) return rc;
   if ((rc = batch_run(&b, nullptr))) return rc;
   CK(cudaMemcpyAsync(out, b.dc.p, sizeof(sherd_candidate) * n_items, cudaMemcpyDeviceToHost,
                      ctx->stream));
