@@ -145,15 +145,26 @@ __device__ K block_select(const K *keys, uint32_t n, uint32_t k, VerShared &sh) 
       if ((key & mask) == prefix) atomicAdd(&sh.hist[(key >> shift) & 255u], 1u);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned kk = sh.kk, cum = 0;
-      int b = 0;
-      for (; b < 255; ++b) {
-        if (cum + sh.hist[b] > kk) break;
-        cum += sh.hist[b];
+    if (threadIdx.x < 32) {
+      // The digit the k-th key has: a warp's prefix sum over the 256 counts, eight
+      // a lane (one thread's walk over them took 4 us a digit, 48 digits an item).
+      const int lane = threadIdx.x;
+      const unsigned kk = sh.kk;
+      unsigned own = 0;
+      for (int j = 0; j < 8; ++j) own += sh.hist[8 * lane + j];
+      unsigned incl = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
       }
-      sh.kk = kk - cum;
-      sh.prefix = prefix | ((unsigned long long)b << shift);
+      if (incl - own <= kk && kk < incl) {  // one lane: k is below the count of the keys
+        unsigned cum = incl - own;
+        int b = 8 * lane;
+        while (cum + sh.hist[b] <= kk) cum += sh.hist[b++];
+        sh.kk = kk - cum;
+        sh.prefix = prefix | ((unsigned long long)b << shift);
+      }
     }
     mask |= 255ULL << shift;
     __syncthreads();
