@@ -2278,32 +2278,39 @@ int drop_small(sherd_ctx *ctx, DBuf<uint8_t> &mask, uint8_t target, double min_a
   return SHERD_OK;
 }
 
-// One radius-ball pass over every representative (k_ball), its shared memory
-// sized to the largest ball by a counting pass (k_ball_size).
+// One radius-ball pass over every representative: a warp each (k_ball_warp), and a
+// block each for the few whose ball is too large for a warp (k_ball_block), run
+// again with room for the largest when even that does not fit.
 int ball_pass(sherd_ctx *ctx, const CloudView &all, const double *cent, const uint32_t *rep,
               uint32_t n_rep, double radius, int mode, const double *normals, const double *areas,
               const uint8_t *frac, double *out3, uint8_t *flag) {
   cudaStream_t s = ctx->stream;
-  const unsigned grid = std::max(1u, std::min(n_rep, unsigned(ctx->sm_count) * 16u));
-  DBuf<uint32_t> mx;
-  CK(mx.alloc(2));
-  CK(cudaMemsetAsync(mx.p, 0, 8, s));
-  k_ball_size<<<std::min(blocks_for(n_rep, 128), unsigned(ctx->sm_count) * 8u), 128, 0, s>>>(
-      all, cent, rep, n_rep, radius, mode, frac, mx.p, mx.p + 1, ctx->d_status);
+  const BallSums sums{mode, normals, areas, frac, out3, flag};
+  DBuf<uint32_t> mx, large;  // the large ones' count, most members, most leaf ranges
+  CK(mx.alloc(3));
+  CK(large.alloc(std::max(n_rep, 1u)));
+  CK(cudaMemsetAsync(mx.p, 0, 12, s));
+  k_ball_warp<<<std::max(1u, std::min(blocks_for(size_t(n_rep) * 32, BALL_WARPS * 32),
+                                      unsigned(ctx->sm_count) * 32u)),
+                BALL_WARPS * 32, 0, s>>>(all, cent, rep, n_rep, radius, sums, large.p, mx.p);
   CK(cudaGetLastError());
-  uint32_t h[2];
-  CK(cudaMemcpyAsync(h, mx.p, 8, cudaMemcpyDeviceToHost, s));
+  uint32_t h[3] = {};
+  CK(cudaMemcpyAsync(h, mx.p, 4, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
-  uint32_t cap = 1;
-  while (cap < h[0]) cap <<= 1;
-  const uint32_t rcap = std::max(1u, h[1]);
-  const size_t bytes = size_t(cap) * 4 + size_t(rcap) * 8;
-  if (bytes > size_t(200) << 10)
-    return fail(ctx, SHERD_E_INVALID, "a radius ball holds more faces than shared memory does");
-  CK(cudaFuncSetAttribute(k_ball, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-  k_ball<<<grid, BALL_BLOCK, bytes, s>>>(all, cent, rep, n_rep, radius, mode, normals, areas, frac,
-                                         out3, flag, cap, rcap, ctx->d_status);
-  CK(cudaGetLastError());
+  for (uint32_t cap = 8192; h[0]; cap = 32768) {
+    const size_t bytes = size_t(32) * BALL_BLOCK + size_t(4) * BALL_BLOCK_STACK + size_t(4) * cap;
+    CK(cudaFuncSetAttribute(k_ball_block, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+    k_ball_block<<<std::min(h[0], unsigned(ctx->sm_count) * 4u), BALL_BLOCK, bytes, s>>>(
+        all, cent, rep, large.p, h[0], radius, sums, cap, mx.p + 1, mx.p + 2);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(h + 1, mx.p + 1, 8, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    uint32_t pow2 = 1;
+    while (pow2 < h[1]) pow2 <<= 1;
+    if (size_t(pow2) * 4 + size_t(std::max(1u, h[2])) * 8 > size_t(200) << 10)
+      return fail(ctx, SHERD_E_INVALID, "a radius ball holds more faces than shared memory does");
+    if (h[1] <= cap) break;
+  }
   return SHERD_OK;
 }
 
