@@ -470,14 +470,20 @@ __global__ void k_uf_roots(uint32_t *parent, const uint8_t *mask, uint8_t target
 }
 
 // One thread per component: its area, summed in face order (the roots were
-// sorted stably, so each run lists its faces ascending).
+// sorted stably, so each run lists its faces ascending), as far as the sum takes
+// to reach min_area: areas are not negative, so it stays there, and whether it
+// does is all that is asked (the shell of a 66 144-face mesh took 1.9 ms to its
+// end).
 __global__ void k_component_areas(const uint32_t *root, const uint32_t *face, uint32_t n,
-                                  const double *areas, double *size) {
+                                  const double *areas, double min_area, double *size) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || root[i] == MISS || (i > 0 && root[i - 1] == root[i])) return;
   double s = 0.0;
   uint32_t j = i;
-  for (; j < n && root[j] == root[i]; ++j) s += areas[face[j]];
+  for (; j < n && root[j] == root[i]; ++j) {
+    s += areas[face[j]];
+    if (s >= min_area) break;
+  }
   size[root[i]] = s;
 }
 

@@ -2271,7 +2271,7 @@ int drop_small(sherd_ctx *ctx, DBuf<uint8_t> &mask, uint8_t target, double min_a
   CK(cudaGetLastError());
   int rc = radix_sort_pairs(ctx, root.p, root2.p, face.p, face2.p, nf, 32);
   if (rc) return rc;
-  k_component_areas<<<blocks_for(nf), 256, 0, s>>>(root2.p, face2.p, nf, areas.p, size.p);
+  k_component_areas<<<blocks_for(nf), 256, 0, s>>>(root2.p, face2.p, nf, areas.p, min_area, size.p);
   k_drop_small<<<blocks_for(nf), 256, 0, s>>>(mask.p, target, nf, parent.p, size.p, min_area);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(s));
