@@ -406,18 +406,24 @@ class Context:
         args = (self.h, v, len(v), f, len(f), frac, float(t), float(macro_inner),
                 float(macro_outer), float(brk_voxel))
         count, n_sub = C.c_uint32(0), C.c_uint32(0)
-        check(self.h, A.lib().sherd_breaklines(*args, 0, None, None, None, None, None, None,
-                                               None, C.byref(n_sub), C.byref(count)))
-        n = count.value
-        out = {"p": np.zeros((n, 3)), "ns": np.zeros((n, 3)), "nf": np.zeros((n, 3)),
-               "f": np.zeros((n, 3)), "dih": np.zeros(n), "valid": np.zeros(n, np.uint8),
-               "sub": np.zeros(max(n, 1), np.uint32)}
-        if n:
-            check(self.h, A.lib().sherd_breaklines(
-                *args, n, ptr(out["p"]), ptr(out["ns"]), ptr(out["nf"]), ptr(out["f"]),
+        # Room for a breakline of the usual length (it grows with the mesh's edge, not its
+        # area); a longer one is refused with its count, and asked for again.
+        room = 256 + 16 * int(len(f) ** 0.5)
+        while True:
+            out = {"p": np.empty((room, 3)), "ns": np.empty((room, 3)), "nf": np.empty((room, 3)),
+                   "f": np.empty((room, 3)), "dih": np.empty(room),
+                   "valid": np.empty(room, np.uint8), "sub": np.empty(room, np.uint32)}
+            rc = A.lib().sherd_breaklines(
+                *args, room, ptr(out["p"]), ptr(out["ns"]), ptr(out["nf"]), ptr(out["f"]),
                 ptr(out["dih"]), ptr(out["valid"]), ptr(out["sub"]), C.byref(n_sub),
-                C.byref(count)))
-        out["sub"] = out["sub"][:n_sub.value].copy()
+                C.byref(count))
+            if rc == A.E_INVALID and count.value > room:
+                room = count.value
+                continue
+            check(self.h, rc)
+            break
+        n = count.value
+        out = {k: a[:n_sub.value if k == "sub" else n].copy() for k, a in out.items()}
         out["valid"] = out["valid"].astype(bool)
         return out
 

@@ -167,7 +167,16 @@ struct BuildBox {
   double lo[3], inv[3];
 };
 
-__global__ void k_morton_tri(const float *v, const uint32_t *f, uint32_t nf, BuildBox box,
+// The Morton codes' box from the bounds.
+__global__ void k_build_box(const unsigned *bounds, BuildBox *box) {
+  const int k = threadIdx.x;
+  if (k >= 3) return;
+  const double lo = fordinv(bounds[k]), hi = fordinv(bounds[3 + k]), ext = hi - lo;
+  box->lo[k] = lo;
+  box->inv[k] = ext > 0.0 ? 1.0 / ext : 0.0;
+}
+
+__global__ void k_morton_tri(const float *v, const uint32_t *f, uint32_t nf, const BuildBox *box,
                              unsigned long long *keys, uint32_t *vals) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nf) return;
@@ -175,15 +184,15 @@ __global__ void k_morton_tri(const float *v, const uint32_t *f, uint32_t nf, Bui
   for (int k = 0; k < 3; ++k)
     c[k] = (double(v[3 * f[3 * i] + k]) + double(v[3 * f[3 * i + 1] + k]) +
             double(v[3 * f[3 * i + 2] + k])) / 3.0;
-  keys[i] = morton3(c[0], c[1], c[2], box.lo, box.inv);
+  keys[i] = morton3(c[0], c[1], c[2], box->lo, box->inv);
   vals[i] = i;
 }
 
-__global__ void k_morton_pts(const double *p, uint32_t n, BuildBox box, unsigned long long *keys,
+__global__ void k_morton_pts(const double *p, uint32_t n, const BuildBox *box, unsigned long long *keys,
                              uint32_t *vals) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  keys[i] = morton3(p[3 * i], p[3 * i + 1], p[3 * i + 2], box.lo, box.inv);
+  keys[i] = morton3(p[3 * i], p[3 * i + 1], p[3 * i + 2], box->lo, box->inv);
   vals[i] = i;
 }
 
@@ -199,9 +208,11 @@ __device__ __forceinline__ int kdelta(const unsigned long long *keys, int n, int
 // Internal node i of n-1: children (leaf primitive k encoded as k | 0x80000000),
 // the primitive range it covers and the parent links.
 __global__ void k_karras(const unsigned long long *keys, int n, int *left, int *right, int *first,
-                         int *last, int *parent_int, int *parent_leaf) {
+                         int *last, int *parent_int, int *parent_leaf, unsigned *flags) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n - 1) return;
+  flags[i] = 0;                     // for k_refit
+  if (i == 0) parent_int[0] = -1;  // the root
   int d = (kdelta(keys, n, i, i + 1) - kdelta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
   int dmin = kdelta(keys, n, i, i - d);
   int lmax = 2;

@@ -232,10 +232,10 @@ Pose16 pose_of(const double *t) {
 // turns the kernels' status bits into an error code.
 int finish(sherd_ctx *ctx, const char *method, size_t items, bool timed) {
   CK(cudaEventRecord(ctx->ev1, ctx->stream));
+  uint32_t st = 0;
+  CK(cudaMemcpyAsync(&st, ctx->d_status, 4, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   CK(cudaGetLastError());
-  uint32_t st = 0;
-  CK(cudaMemcpy(&st, ctx->d_status, 4, cudaMemcpyDeviceToHost));
   MethodStats &m = ctx->stats[method];
   m.calls += 1;
   m.items += items;
@@ -351,11 +351,12 @@ struct sherd_pair {
 namespace {
 
 // Builds the LBVH over f32 triangles (TRI) or f64 points (!TRI) already on the
-// device; fills nodes, the sorted slot order and the root description.
+// device; fills nodes and the sorted slot order. Nothing here or in what calls it
+// waits for the device (buffers are freed in stream order): the entry points that
+// hand a tree to the caller wait at their end.
 template <bool TRI>
 int build_lbvh(sherd_ctx *ctx, const float *d_v, uint32_t nv, const uint32_t *d_f, const double *d_p,
-               uint32_t n, float pad, int leaf_max, DBuf<BNode> &nodes, DBuf<uint32_t> &sorted,
-               float lo[3], float hi[3]) {
+               uint32_t n, float pad, int leaf_max, DBuf<BNode> &nodes, DBuf<uint32_t> &sorted) {
   cudaStream_t s = ctx->stream;
   DBuf<unsigned> bounds;
   CK(bounds.alloc(6));
@@ -366,17 +367,10 @@ int build_lbvh(sherd_ctx *ctx, const float *d_v, uint32_t nv, const uint32_t *d_
   else
     k_bounds_f64<<<std::min(blocks_for(n), 1024u), 256, 0, s>>>(d_p, n, bounds.p);
   CK(cudaGetLastError());
-  unsigned hb[6];
-  CK(cudaMemcpyAsync(hb, bounds.p, sizeof hb, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  BuildBox box;
-  for (int k = 0; k < 3; ++k) {
-    lo[k] = fordinv(hb[k]);
-    hi[k] = fordinv(hb[3 + k]);
-    box.lo[k] = lo[k];
-    double ext = double(hi[k]) - double(lo[k]);
-    box.inv[k] = ext > 0.0 ? 1.0 / ext : 0.0;
-  }
+  DBuf<BuildBox> box;
+  CK(box.alloc(1));
+  k_build_box<<<1, 32, 0, s>>>(bounds.p, box.p);
+  CK(cudaGetLastError());
   DBuf<unsigned long long> keys, keys2;
   DBuf<uint32_t> vals;
   CK(keys.alloc(n));
@@ -384,9 +378,9 @@ int build_lbvh(sherd_ctx *ctx, const float *d_v, uint32_t nv, const uint32_t *d_
   CK(vals.alloc(n));
   CK(sorted.alloc(n));
   if (TRI)
-    k_morton_tri<<<blocks_for(n), 256, 0, s>>>(d_v, d_f, n, box, keys.p, vals.p);
+    k_morton_tri<<<blocks_for(n), 256, 0, s>>>(d_v, d_f, n, box.p, keys.p, vals.p);
   else
-    k_morton_pts<<<blocks_for(n), 256, 0, s>>>(d_p, n, box, keys.p, vals.p);
+    k_morton_pts<<<blocks_for(n), 256, 0, s>>>(d_p, n, box.p, keys.p, vals.p);
   CK(cudaGetLastError());
   size_t temp_bytes = 0;
   CK(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys.p, keys2.p, vals.p, sorted.p,
@@ -397,7 +391,6 @@ int build_lbvh(sherd_ctx *ctx, const float *d_v, uint32_t nv, const uint32_t *d_
                                      0, 63, s));
   if (int(n) <= leaf_max) {
     nodes.reset();
-    CK(cudaStreamSynchronize(s));
     return SHERD_OK;
   }
   int ni = int(n) - 1;
@@ -413,10 +406,8 @@ int build_lbvh(sherd_ctx *ctx, const float *d_v, uint32_t nv, const uint32_t *d_
   CK(flags.alloc(ni));
   CK(ibox.alloc(size_t(6) * ni));
   CK(nodes.alloc(ni));
-  CK(cudaMemsetAsync(flags.p, 0, sizeof(unsigned) * ni, s));
-  CK(cudaMemsetAsync(pint.p, 0xFF, sizeof(int) * ni, s));  // root's parent is -1
   k_karras<<<blocks_for(ni), 256, 0, s>>>(keys2.p, int(n), left.p, right.p, first.p, last.p, pint.p,
-                                          pleaf.p);
+                                          pleaf.p, flags.p);
   CK(cudaGetLastError());
   k_refit<TRI><<<blocks_for(n), 256, 0, s>>>(d_v, d_f, d_p, sorted.p, int(n), left.p, right.p,
                                              pint.p, pleaf.p, flags.p, ibox.p);
@@ -424,7 +415,6 @@ int build_lbvh(sherd_ctx *ctx, const float *d_v, uint32_t nv, const uint32_t *d_
   k_emit<TRI><<<blocks_for(ni), 256, 0, s>>>(d_v, d_f, d_p, sorted.p, int(n), left.p, right.p,
                                              first.p, last.p, ibox.p, pad, leaf_max, nodes.p);
   CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(s));
   return SHERD_OK;
 }
 
@@ -439,13 +429,11 @@ int mesh_build(sherd_ctx *ctx, sherd_mesh *m) {
   double mag = 1.0;
   for (float x : m->hv) mag = std::max(mag, double(std::fabs(x)));
   float pad = float(1e-5 * mag);
-  float lo[3], hi[3];
-  rc = build_lbvh<true>(ctx, dv.p, nv, df.p, nullptr, nf, pad, TRI_LEAF, m->nodes, sorted, lo, hi);
+  rc = build_lbvh<true>(ctx, dv.p, nv, df.p, nullptr, nf, pad, TRI_LEAF, m->nodes, sorted);
   if (rc) return rc;
   CK(m->tri.alloc(size_t(3) * nf));
   k_store_tris<<<blocks_for(nf), 256, 0, ctx->stream>>>(dv.p, df.p, sorted.p, nf, m->tri.p);
   CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(ctx->stream));
   // The exact vertex box of RayScene::aabb (bvh.rs:182-185).
   float vlo[3] = {f_inf(), f_inf(), f_inf()}, vhi[3] = {-f_inf(), -f_inf(), -f_inf()};
   for (uint32_t i = 0; i < nv; ++i)
@@ -462,9 +450,13 @@ int mesh_build(sherd_ctx *ctx, sherd_mesh *m) {
                       double(a[2] - b[2]) * (a[2] - b[2]));
   }
   edge = std::max(edge / std::max<uint32_t>(nf, 1), 1e-6);
+  AxisGrid grids[3] = {};
+  DBuf<unsigned> count[3], dtotal;
+  uint32_t total[3] = {};
+  CK(dtotal.alloc(3));
   for (int axis = 0; axis < 3; ++axis) {
     int au = (axis + 1) % 3, av = (axis + 2) % 3;
-    AxisGrid g{};
+    AxisGrid &g = grids[axis];
     double lo_u = double(vlo[au]) - 2.0 * pad, lo_v = double(vlo[av]) - 2.0 * pad;
     double ext_u = double(vhi[au]) - lo_u + 2.0 * pad, ext_v = double(vhi[av]) - lo_v + 2.0 * pad;
     double cell = edge;
@@ -475,30 +467,34 @@ int mesh_build(sherd_ctx *ctx, sherd_mesh *m) {
     g.nu = uint32_t(ext_u / cell) + 2;
     g.nv = uint32_t(ext_v / cell) + 2;
     size_t cells = size_t(g.nu) * g.nv;
-    DBuf<unsigned> count;
-    CK(count.alloc(cells + 1));
-    CK(cudaMemsetAsync(count.p, 0, sizeof(unsigned) * (cells + 1), ctx->stream));
-    k_grid_count<<<blocks_for(nf), 256, 0, ctx->stream>>>(m->tri.p, nf, axis, g, pad, count.p);
+    CK(count[axis].alloc(cells + 1));
+    CK(cudaMemsetAsync(count[axis].p, 0, sizeof(unsigned) * (cells + 1), ctx->stream));
+    k_grid_count<<<blocks_for(nf), 256, 0, ctx->stream>>>(m->tri.p, nf, axis, g, pad, count[axis].p);
     CK(cudaGetLastError());
     CK(m->gstart[axis].alloc(cells + 1));
     size_t temp_bytes = 0;
-    CK(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, count.p, m->gstart[axis].p, int(cells + 1),
+    CK(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, count[axis].p, m->gstart[axis].p, int(cells + 1),
                                      ctx->stream));
     DBuf<unsigned char> temp;
     CK(temp.alloc(temp_bytes));
-    CK(cub::DeviceScan::ExclusiveSum(temp.p, temp_bytes, count.p, m->gstart[axis].p, int(cells + 1),
+    CK(cub::DeviceScan::ExclusiveSum(temp.p, temp_bytes, count[axis].p, m->gstart[axis].p, int(cells + 1),
                                      ctx->stream));
-    uint32_t total = 0;
-    CK(cudaMemcpyAsync(&total, m->gstart[axis].p + cells, 4, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    CK(m->grect[axis].alloc(std::max<uint32_t>(total, 1)));
-    CK(m->gtri[axis].alloc(3 * size_t(std::max<uint32_t>(total, 1))));
-    CK(cudaMemcpyAsync(count.p, m->gstart[axis].p, sizeof(unsigned) * cells, cudaMemcpyDeviceToDevice,
+    CK(cudaMemcpyAsync(dtotal.p + axis, m->gstart[axis].p + cells, 4, cudaMemcpyDeviceToDevice,
                        ctx->stream));
-    k_grid_fill<<<blocks_for(nf), 256, 0, ctx->stream>>>(m->tri.p, nf, axis, g, pad, count.p,
+  }
+  // The entries' numbers, to size them: the one wait of a build.
+  CK(cudaMemcpyAsync(total, dtotal.p, sizeof total, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  for (int axis = 0; axis < 3; ++axis) {
+    AxisGrid &g = grids[axis];
+    const size_t entries = std::max<uint32_t>(total[axis], 1);
+    CK(m->grect[axis].alloc(entries));
+    CK(m->gtri[axis].alloc(3 * entries));
+    CK(cudaMemcpyAsync(count[axis].p, m->gstart[axis].p, sizeof(unsigned) * size_t(g.nu) * g.nv,
+                       cudaMemcpyDeviceToDevice, ctx->stream));
+    k_grid_fill<<<blocks_for(nf), 256, 0, ctx->stream>>>(m->tri.p, nf, axis, g, pad, count[axis].p,
                                                         m->grect[axis].p, m->gtri[axis].p);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(ctx->stream));
     g.start = m->gstart[axis].p;
     g.rect = m->grect[axis].p;
     g.tri = m->gtri[axis].p;
@@ -547,9 +543,7 @@ int mesh_build(sherd_ctx *ctx, sherd_mesh *m) {
 int cloud_build_dev(sherd_ctx *ctx, const double *dp, const double *dn, uint32_t np, float pad,
                     sherd_cloud *c) {
   DBuf<uint32_t> sorted;
-  float lo[3], hi[3];
-  int rc = build_lbvh<false>(ctx, nullptr, 0, nullptr, dp, np, pad, POINT_LEAF, c->nodes, sorted,
-                             lo, hi);
+  int rc = build_lbvh<false>(ctx, nullptr, 0, nullptr, dp, np, pad, POINT_LEAF, c->nodes, sorted);
   if (rc) return rc;
   CK(c->pts.alloc(np));
   if (dn) CK(c->nrm.alloc(np));
@@ -562,7 +556,6 @@ int cloud_build_dev(sherd_ctx *ctx, const double *dp, const double *dn, uint32_t
     k_widen<<<blocks_for(np - 1), 256, 0, ctx->stream>>>(c->nodes.p, int(np - 1), c->wide.p);
     CK(cudaGetLastError());
   }
-  CK(cudaStreamSynchronize(ctx->stream));
   c->ctx = ctx;
   CloudView &v = c->view;
   v.nodes = c->nodes.p;
@@ -604,6 +597,13 @@ ConeConsts cone_consts() {
   return cc;
 }
 
+// The bits that indices below n have.
+int bits_below(uint32_t n) {
+  int bits = 1;
+  while (bits < 32 && (uint64_t(1) << bits) < uint64_t(n)) ++bits;
+  return bits;
+}
+
 template <typename K, typename V>
 int radix_sort_pairs(sherd_ctx *ctx, const K *kin, K *kout, const V *vin, V *vout, uint32_t n,
                      int end_bit) {
@@ -614,7 +614,6 @@ int radix_sort_pairs(sherd_ctx *ctx, const K *kin, K *kout, const V *vin, V *vou
   CK(tmp.alloc(bytes));
   CK(cub::DeviceRadixSort::SortPairs(tmp.p, bytes, kin, kout, vin, vout, int(n), 0, end_bit,
                                      ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
   return SHERD_OK;
 }
 
@@ -859,6 +858,7 @@ int sherd_mesh_upload(sherd_ctx *ctx, const float *v, uint32_t nv, const uint32_
     delete m;
     return rc;
   }
+  CK(cudaStreamSynchronize(ctx->stream));
   *out = m;
   return SHERD_OK;
 }
@@ -880,6 +880,7 @@ int sherd_mesh_subset(sherd_ctx *ctx, const sherd_mesh *mesh, const uint8_t *kee
     delete m;
     return rc;
   }
+  CK(cudaStreamSynchronize(ctx->stream));
   *out = m;
   return SHERD_OK;
 }
@@ -1202,6 +1203,7 @@ int sherd_cloud_upload(sherd_ctx *ctx, const double *points, const double *norma
     delete c;
     return rc;
   }
+  CK(cudaStreamSynchronize(ctx->stream));
   *out = c;
   return SHERD_OK;
 }
@@ -2274,7 +2276,6 @@ int drop_small(sherd_ctx *ctx, DBuf<uint8_t> &mask, uint8_t target, double min_a
   k_component_areas<<<blocks_for(nf), 256, 0, s>>>(root2.p, face2.p, nf, areas.p, min_area, size.p);
   k_drop_small<<<blocks_for(nf), 256, 0, s>>>(mask.p, target, nf, parent.p, size.p, min_area);
   CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(s));
   return SHERD_OK;
 }
 
@@ -2342,8 +2343,7 @@ int vertex_normals_dev(sherd_ctx *ctx, const double *dv, uint32_t nv, const uint
     CK(face2.alloc(nc));
     k_incidence<<<blocks_for(nc), 256, 0, s>>>(df, nc, key.p, face.p);
     CK(cudaGetLastError());
-    int bits = 1;  // vertex ids are below nv <= 2^bits
-    while (bits < 32 && (uint64_t(1) << bits) < uint64_t(nv)) ++bits;
+    const int bits = bits_below(nv);
     // LSD radix sort is stable: each vertex keeps its faces in ascending order.
     int rc = radix_sort_pairs(ctx, key.p, key2.p, face.p, face2.p, nc, bits);
     if (rc) return rc;
@@ -2425,10 +2425,10 @@ int sherd_segment(sherd_ctx *ctx, const sherd_mesh *mesh, const double *v, uint3
     CK(tmp.alloc(bytes));
     CK(cub::DeviceSelect::Flagged(tmp.p, bytes, idx2.p, heads.p, rep_unsorted.p, nrep_dev.p,
                                   int(nf), s));
-    CK(cudaStreamSynchronize(s));
   }
   uint32_t n_rep = 0;
-  CK(cudaMemcpy(&n_rep, nrep_dev.p, 4, cudaMemcpyDeviceToHost));
+  CK(cudaMemcpyAsync(&n_rep, nrep_dev.p, 4, cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
   inf.n_rep = n_rep;
   CK(rep.alloc(n_rep));
   {
@@ -2437,7 +2437,6 @@ int sherd_segment(sherd_ctx *ctx, const sherd_mesh *mesh, const double *v, uint3
     DBuf<unsigned char> tmp;
     CK(tmp.alloc(bytes));
     CK(cub::DeviceRadixSort::SortKeys(tmp.p, bytes, rep_unsorted.p, rep.p, int(n_rep), 0, 32, s));
-    CK(cudaStreamSynchronize(s));
   }
   DBuf<double> rep_pts;
   CK(rep_pts.alloc(size_t(3) * n_rep));
@@ -2497,7 +2496,7 @@ int sherd_segment(sherd_ctx *ctx, const sherd_mesh *mesh, const double *v, uint3
   CK(ep2.alloc(m));
   k_edge_keys<<<blocks_for(nf), 256, 0, s>>>(df.p, nf, ek.p, ep.p);
   CK(cudaGetLastError());
-  if ((rc = radix_sort_pairs(ctx, ek.p, ek2.p, ep.p, ep2.p, m, 64))) return rc;
+  if ((rc = radix_sort_pairs(ctx, ek.p, ek2.p, ep.p, ep2.p, m, 32 + bits_below(nv)))) return rc;
   CK(fa.alloc(n_pairs));
   CK(fb.alloc(n_pairs));
   k_face_pairs<<<blocks_for(m), 256, 0, s>>>(ek2.p, ep2.p, m, nf, fa.p, fb.p);
@@ -2540,12 +2539,16 @@ int sherd_segment(sherd_ctx *ctx, const sherd_mesh *mesh, const double *v, uint3
   CK(cudaMemsetAsync(cand.p, 0, nf, s));
   DBuf<uint32_t> flipped;
   CK(flipped.alloc(1));
-  for (int pass = 0; pass < 60; ++pass) {
+  // A pass without flips leaves everything as it is, and so do the passes after
+  // it, so the host looks every few passes.
+  constexpr int GROW_PASSES = 60, GROW_LOOK = 4;
+  for (int pass = 0; pass < GROW_PASSES; ++pass) {
     CK(cudaMemsetAsync(flipped.p, 0, 4, s));
     k_grow_candidates<<<blocks_for(n_pairs), 256, 0, s>>>(fa.p, fb.p, n_pairs, frac.p, cand.p);
     k_grow_flip<<<blocks_for(nf), 256, 0, s>>>(cand.p, frac.p, nf, normals.p, ref.p, has_ref.p,
                                                cos_grow, flipped.p);
     CK(cudaGetLastError());
+    if (pass % GROW_LOOK != GROW_LOOK - 1) continue;
     uint32_t any = 0;
     CK(cudaMemcpyAsync(&any, flipped.p, 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -3065,7 +3068,6 @@ int macro_normals(sherd_ctx *ctx, const double *p, uint32_t n, const double *cen
     if ((r = ball_pass(ctx, sub.view, p, q_idx, nq, outer, BALL_NORMALS, nn.p, a.p, nullptr, res3,
                        flag.p)))
       return r;
-    CK(cudaStreamSynchronize(s));
     return SHERD_OK;
   };
   CK(queries.alloc(n));
@@ -3140,7 +3142,7 @@ int sherd_breaklines(sherd_ctx *ctx, const double *v, uint32_t nv, const uint32_
   CK(ep2.alloc(m));
   k_edge_keys<<<blocks_for(nf), 256, 0, s>>>(df.p, nf, ek.p, ep.p);
   CK(cudaGetLastError());
-  if ((rc = radix_sort_pairs(ctx, ek.p, ek2.p, ep.p, ep2.p, m, 64))) return rc;
+  if ((rc = radix_sort_pairs(ctx, ek.p, ek2.p, ep.p, ep2.p, m, 32 + bits_below(nv)))) return rc;
   CK(fa.alloc(n_pairs));
   CK(fb.alloc(n_pairs));
   k_face_pairs<<<blocks_for(m), 256, 0, s>>>(ek2.p, ep2.p, m, nf, fa.p, fb.p);
