@@ -1179,7 +1179,7 @@ int sherd_cone_votes(sherd_ctx *ctx, const sherd_mesh *mesh, const double *centr
       (rc = upload(ctx, dns, ns, size_t(3) * nf)) || (rc = upload(ctx, dh, hit_normals, size_t(3) * nf)))
     return rc;
   CK(dg.alloc(nf));
-  k_cone_votes<<<blocks_for(nf, 128), 128, 0, ctx->stream>>>(mesh->view, dc.p, dn.p, dns.p, dh.p, nf,
+  k_cone_votes<<<blocks_for(nf, 32), CONE_BLOCK, 0, ctx->stream>>>(mesh->view, dc.p, dn.p, dns.p, dh.p, nf,
                                                             thick, cc, dg.p, ctx->d_status);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(good, dg.p, nf, cudaMemcpyDeviceToHost, ctx->stream));
@@ -2465,7 +2465,7 @@ int sherd_segment(sherd_ctx *ctx, const sherd_mesh *mesh, const double *v, uint3
   // 3.4.3 the cone vote.
   CK(good.alloc(nf));
   CK(frac.alloc(nf));
-  k_cone_votes<<<blocks_for(nf, 128), 128, 0, s>>>(mesh->view, cent.p, normals.p, ns.p,
+  k_cone_votes<<<blocks_for(nf, 32), CONE_BLOCK, 0, s>>>(mesh->view, cent.p, normals.p, ns.p,
                                                   sp.smoothed_hit_normal ? ns.p : normals.p, nf,
                                                   thick, cone_consts(), good.p, ctx->d_status);
   k_votes_to_frac<<<blocks_for(nf), 256, 0, s>>>(good.p, nf, inf.votes, frac.p);
