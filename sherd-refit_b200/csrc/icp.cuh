@@ -545,8 +545,11 @@ __device__ __noinline__ int nearest_guarded(const CloudView &c, double qx, doubl
   }
   const float qc[3] = {float(qx), float(qy), float(qz)};
   auto leaf = [&](int first, int count) {
-    for (int s = first; s < first + count; ++s)
-      if (s != best_s) score(s, ldg4(c.pts + s));
+    // Both points of a leaf are read before either is scored.
+    static_assert(POINT_LEAF <= 2, "a leaf holds one or two points");
+    const double4 p0 = ldg4(c.pts + first), p1 = ldg4(c.pts + first + (count - 1));
+    if (first != best_s) score(first, p0);
+    if (count > 1 && first + 1 != best_s) score(first + 1, p1);
   };
   if (c.root_leaf)
     leaf(0, c.root_leaf);
