@@ -107,7 +107,10 @@ __device__ __forceinline__ void add_twist(double *acc, int o, const double *p, c
 
 // Unit u = (pose * n_edges + edge) * 3 + kind; kind 0 plane, 1 side B, 2 side A.
 // values: n_poses * n_edges * ADJ_VALUES; grads: the same * 6.
-__global__ void __launch_bounds__(ADJ_BLOCK) k_adjoint(const PairView *edges, uint32_t n_edges,
+// Four blocks of 256 an SM (64 registers; the pose is read from shared memory): the
+// searches are a chain of loads, and the two blocks that the compiler's own 126
+// registers left took 2.87 ms for 64 poses of a 6-fragment pot, three 2.50, four 2.37.
+__global__ void __launch_bounds__(ADJ_BLOCK, 4) k_adjoint(const PairView *edges, uint32_t n_edges,
                                                        const double *poses, const double *inverses,
                                                        AdjointConsts kc, double *values,
                                                        double *grads, uint32_t *status) {
@@ -118,9 +121,7 @@ __global__ void __launch_bounds__(ADJ_BLOCK) k_adjoint(const PairView *edges, ui
   const PairView &pr = edges[e];
   if (threadIdx.x < 12) s_m[threadIdx.x] = (kind == 2 ? inverses : poses)[16 * size_t(pe) + threadIdx.x];
   __syncthreads();
-  double m[12];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) m[k] = s_m[k];
+  const double *m = s_m;
   double acc[ADJ_SUMS];
 #pragma unroll
   for (int k = 0; k < ADJ_SUMS; ++k) acc[k] = 0.0;
