@@ -1059,21 +1059,18 @@ __device__ __forceinline__ bool min_step(MinWalk &w, bool active, int *stack_n, 
     st |= ST_STACK;
     active = false;
   }
-  int next = -1, leaf[2] = {0, 0};
-  uint32_t faces[2] = {0, 0};
+  int next = -1;
+  uint32_t first = 0, faces = 0;
   if (active) {
     const Child2 n = load_node(w.m->nodes, w.node);
     const float pc[3] = {w.p.x, w.p.y, w.p.z};
     const float k[2] = {box_dist2(n.lo0, n.hi0, pc), box_dist2(n.lo1, n.hi1, pc)};
     const bool in0 = k[0] <= w.bound2, in1 = k[1] <= w.bound2;
-    if (in0 && n.cnt[0]) {
-      leaf[0] = n.ref[0];
-      faces[0] = n.cnt[0];
-    }
-    if (in1 && n.cnt[1]) {
-      leaf[1] = n.ref[1];
-      faces[1] = n.cnt[1];
-    }
+    // The leaves of a node are one run of slots (the left one's end where the
+    // right one's begin).
+    const bool leaf0 = in0 && n.cnt[0], leaf1 = in1 && n.cnt[1];
+    first = leaf0 ? n.ref[0] : n.ref[1];
+    faces = (leaf0 ? n.cnt[0] : 0) + (leaf1 ? n.cnt[1] : 0);
     const bool go0 = in0 && !n.cnt[0], go1 = in1 && !n.cnt[1];
     if (go0 && go1) {
       const bool second = k[1] < k[0];
@@ -1088,11 +1085,9 @@ __device__ __forceinline__ bool min_step(MinWalk &w, bool active, int *stack_n, 
       next = go0 ? n.ref[0] : n.ref[1];
     }
   }
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    if (!__any_sync(0xffffffffu, faces[c] != 0)) continue;
-    const float d = warp_leaves(w.m, w.p, leaf[c], faces[c], slot);
-    if (faces[c]) min_found(w, d);
+  if (__any_sync(0xffffffffu, faces != 0)) {
+    const float d = warp_leaves(w.m, w.p, first, faces, slot);
+    if (faces) min_found(w, d);
   }
   if (!active) return false;
   if ((w.visits & (MIN_LOOK - 1)) == 0) min_look(w);

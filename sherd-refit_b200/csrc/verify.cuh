@@ -18,6 +18,7 @@
 #pragma once
 
 #include "icp.cuh"
+#include "walk.cuh"
 
 namespace sherd {
 
@@ -76,6 +77,8 @@ struct VerShared {
   unsigned cnt[8];
   unsigned best_key;
   unsigned deep_key;
+  unsigned next;  // the next query of one_side
+  WalkSlots<false> walk[32];
   unsigned cells[MAX_CELL_WORDS];
 };
 
@@ -194,28 +197,33 @@ __device__ __noinline__ void one_side(const double4 *pts, uint32_t n, const doub
                          double area, const sherd_scales &sc, unsigned *scratch, VerShared &sh,
                          double &tight, double &gap, double &contact, uint32_t &status) {
   if (threadIdx.x < 3) sh.cnt[threadIdx.x] = 0;
+  if (threadIdx.x == 0) sh.next = 0;
   __syncthreads();
-  float window = float(sc.facing);
-  unsigned facing = 0, tight_n = 0, touching = 0;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    double4 q = ldg4(pts + i);
-    double x, y, z;
-    apply_pose(pose, q.x, q.y, q.z, x, y, z);
-    float d = mesh_distance(scene, narrow3(x, y, z), window, status);
-    double dd = d == f_inf() ? d_inf() : double(d);
-    if (dd < 2.0 * sc.tight) ++touching;
-    if (dd < sc.facing) {
-      ++facing;
-      if (dd < sc.tight) ++tight_n;
-      unsigned slot = atomicAdd(&sh.cnt[0], 1u);
-      scratch[slot] = f2key(d);
-    }
-  }
+  const float window = float(sc.facing);
+  unsigned tight_n = 0, touching = 0;
+  face_walks<false, false>(
+      &sh.next, n, sh.walk[threadIdx.x >> 5],
+      [&](uint32_t i, FaceWalk &w) {
+        double4 q = ldg4(pts + i);
+        double x, y, z;
+        apply_pose(pose, q.x, q.y, q.z, x, y, z);
+        return walk_start<false>(w, &scene, narrow3(x, y, z), window);
+      },
+      [&](uint32_t, const FaceWalk &w) {
+        const float d = w.best;
+        const double dd = d == f_inf() ? d_inf() : double(d);
+        if (dd < 2.0 * sc.tight) ++touching;
+        if (dd < sc.facing) {
+          if (dd < sc.tight) ++tight_n;
+          unsigned slot = atomicAdd(&sh.cnt[0], 1u);
+          scratch[slot] = f2key(d);
+        }
+      },
+      status);
   atomicAdd(&sh.cnt[1], tight_n);
   atomicAdd(&sh.cnt[2], touching);
   __syncthreads();
   unsigned nf = sh.cnt[0], nt = sh.cnt[1], nto = sh.cnt[2];
-  (void)facing;
   __syncthreads();
   if (nf < 20) {
     tight = 0.0;
