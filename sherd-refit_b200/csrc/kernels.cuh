@@ -795,8 +795,9 @@ __device__ __forceinline__ uint32_t warp_crossings(const MeshView *m, F3 p, int 
                                                    unsigned *par_word) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
+  const unsigned long long tri = reinterpret_cast<unsigned long long>(active ? m->tri : nullptr);
   uint32_t b = 0, len = 0;
-  unsigned long long rect = 0, tri = 0;
+  unsigned long long rect = 0, slot = 0;
   if (active && m->nf) {
     const AxisGrid &g = m->grid[axis];
     float pc[3] = {p.x, p.y, p.z};
@@ -807,7 +808,7 @@ __device__ __forceinline__ uint32_t warp_crossings(const MeshView *m, F3 p, int 
       b = __ldg(g.start + cell);
       len = __ldg(g.start + cell + 1) - b;
       rect = reinterpret_cast<unsigned long long>(g.rect);
-      tri = reinterpret_cast<unsigned long long>(g.tri);
+      slot = reinterpret_cast<unsigned long long>(g.slot);
     }
   }
   uint32_t incl = len;
@@ -830,6 +831,7 @@ __device__ __forceinline__ uint32_t warp_crossings(const MeshView *m, F3 p, int 
                 qz = __shfl_sync(FULL, p.z, j);
     const uint32_t bj = __shfl_sync(FULL, b, j), oj = __shfl_sync(FULL, off, j);
     const float4 *rj = reinterpret_cast<const float4 *>(__shfl_sync(FULL, rect, j));
+    const uint32_t *sj = reinterpret_cast<const uint32_t *>(__shfl_sync(FULL, slot, j));
     const float4 *tj = reinterpret_cast<const float4 *>(__shfl_sync(FULL, tri, j));
     if (w < total) {
       const size_t k = size_t(bj) + (w - oj);
@@ -837,9 +839,10 @@ __device__ __forceinline__ uint32_t warp_crossings(const MeshView *m, F3 p, int 
       const float qu = qc[(axis + 1) % 3], qv = qc[(axis + 2) % 3];
       const float4 r = __ldg(rj + k);
       if (!(qu < r.x || qu > r.y || qv < r.z || qv > r.w)) {
-        const float4 t0 = __ldg(tj + 3 * k), t1 = __ldg(tj + 3 * k + 1), t2 = __ldg(tj + 3 * k + 2);
-        if (moller_trumbore_edges({qx, qy, qz}, d, {t0.x, t0.y, t0.z}, {t1.x, t1.y, t1.z},
-                                  {t2.x, t2.y, t2.z}) >= 0.0f)
+        const float4 *t = tj + 3 * size_t(__ldg(sj + k));
+        const float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t + 2);
+        if (moller_trumbore_edges({qx, qy, qz}, d, {a.x, a.y, a.z}, {b.x - a.x, b.y - a.y, b.z - a.z},
+                                  {c.x - a.x, c.y - a.y, c.z - a.z}) >= 0.0f)
           atomicXor(par_word, 1u << j);
       }
     }

@@ -46,7 +46,7 @@ struct __align__(16) WNode {
 struct AxisGrid {
   const uint32_t *start;  // nu * nv + 1 offsets into the entry arrays
   const float4 *rect;     // per entry: the face's padded projected rectangle (u0, u1, v0, v1)
-  const float4 *tri;      // per entry, 3 float4: v0, e1 = v1 - v0, e2 = v2 - v0 (f32)
+  const uint32_t *slot;   // per entry: the face's sorted slot
   float lo_u, lo_v, inv_cell;
   uint32_t nu, nv;
 };
@@ -443,10 +443,11 @@ __global__ void k_grid_count(const float4 *tri, uint32_t nf, int axis, AxisGrid 
     for (int v = v0; v <= v1; ++v) atomicAdd(&count[size_t(u) * g.nv + v], 1u);
 }
 
-// Writes every face's entries: its padded projected rectangle and its vertex
-// and edges, so the parity test reads one contiguous run per cell.
+// Writes every face's entries: its padded projected rectangle and its slot. The
+// parity test reads a cell's rectangles as one run, and the triangle itself
+// only for the few entries whose rectangle holds the point.
 __global__ void k_grid_fill(const float4 *tri, uint32_t nf, int axis, AxisGrid g, float pad,
-                            unsigned *cursor, float4 *rect, float4 *edge) {
+                            unsigned *cursor, float4 *rect, uint32_t *slot) {
   uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nf) return;
   int u0, u1, v0, v1;
@@ -458,16 +459,11 @@ __global__ void k_grid_fill(const float4 *tri, uint32_t nf, int axis, AxisGrid g
                          __fadd_ru(fmaxf(ac[au], fmaxf(bc[au], cc[au])), pad),
                          __fsub_rd(fminf(ac[av], fminf(bc[av], cc[av])), pad),
                          __fadd_ru(fmaxf(ac[av], fmaxf(bc[av], cc[av])), pad));
-  float4 t0 = make_float4(a.x, a.y, a.z, 0.0f);
-  float4 t1 = make_float4(b.x - a.x, b.y - a.y, b.z - a.z, 0.0f);
-  float4 t2 = make_float4(c.x - a.x, c.y - a.y, c.z - a.z, 0.0f);
   for (int u = u0; u <= u1; ++u)
     for (int v = v0; v <= v1; ++v) {
       unsigned k = atomicAdd(&cursor[size_t(u) * g.nv + v], 1u);
       rect[k] = r;
-      edge[3 * size_t(k)] = t0;
-      edge[3 * size_t(k) + 1] = t1;
-      edge[3 * size_t(k) + 2] = t2;
+      slot[k] = s;
     }
 }
 

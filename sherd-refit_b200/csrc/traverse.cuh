@@ -167,11 +167,10 @@ __device__ __noinline__ uint32_t crossings_axis(const MeshView &m, F3 p, int axi
   for (uint32_t k = b; k < e; ++k) {
     float4 r = __ldg(g.rect + k);
     if (pu < r.x || pu > r.y || pv < r.z || pv > r.w) continue;
-    float4 t0 = __ldg(g.tri + 3 * size_t(k)), t1 = __ldg(g.tri + 3 * size_t(k) + 1),
-           t2 = __ldg(g.tri + 3 * size_t(k) + 2);
-    if (moller_trumbore_edges(p, d, {t0.x, t0.y, t0.z}, {t1.x, t1.y, t1.z}, {t2.x, t2.y, t2.z}) >=
-        0.0f)
-      ++hits;
+    F3 a, b1, c;
+    uint32_t id;
+    tri_at(m, __ldg(g.slot + k), a, b1, c, id);
+    if (moller_trumbore_edges(p, d, a, sub(b1, a), sub(c, a)) >= 0.0f) ++hits;
   }
   (void)status;
   return hits;
