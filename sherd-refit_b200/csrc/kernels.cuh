@@ -22,15 +22,37 @@ __global__ void k_first_hit(MeshView m, const float *org, const float *dir, uint
   if (st) atomicOr(status, st);
 }
 
-__global__ void k_bounded_all(MeshView m, const double *pts, uint32_t n, Pose16 pose, float window,
-                              double *out, uint32_t *status) {
-  uint32_t st = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double x, y, z;
-    apply_pose(pose.m, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], x, y, z);
-    float d = mesh_distance(m, {float(x), float(y), float(z)}, window, st);
-    out[i] = d == f_inf() ? d_inf() : double(d);
-  }
+// The block's share [first, first + count) of n queries.
+__device__ __forceinline__ uint32_t block_share(uint32_t n, uint32_t &first) {
+  const uint32_t per = (n + gridDim.x - 1) / gridDim.x;
+  first = uint32_t(min((unsigned long long)per * blockIdx.x, (unsigned long long)n));
+  return min(per, n - first);
+}
+
+// Bound by the latency of the walks: a lane's faces shared by its warp, 25,000
+// queries 136 -> 66 us (a thread per query with its own loop over a leaf's faces).
+__global__ void __launch_bounds__(128) k_bounded_all(const __grid_constant__ MeshView m,
+                                                     const double *pts, uint32_t n,
+                                                     const __grid_constant__ Pose16 pose,
+                                                     float window, double *out, uint32_t *status) {
+  __shared__ unsigned next;
+  __shared__ WalkSlots<false> slots[4];
+  if (threadIdx.x == 0) next = 0;
+  __syncthreads();
+  uint32_t st = 0, first;
+  const uint32_t count = block_share(n, first);
+  face_walks<false, false>(
+      &next, count, slots[threadIdx.x >> 5],
+      [&](uint32_t k, FaceWalk &w) {
+        const size_t i = first + k;
+        double x, y, z;
+        apply_pose(pose.m, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], x, y, z);
+        return walk_start<false>(w, &m, {float(x), float(y), float(z)}, window);
+      },
+      [&](uint32_t k, const FaceWalk &w) {
+        out[size_t(first) + k] = w.best == f_inf() ? d_inf() : double(w.best);
+      },
+      st);
   if (st) atomicOr(status, st);
 }
 
@@ -45,22 +67,6 @@ __global__ void k_bounded_min(MeshView m, const double *pts, uint32_t n, Pose16 
     float window = key2f(*((volatile unsigned *)best_key));
     float d = mesh_distance(m, {float(x), float(y), float(z)}, window, st);
     if (d != f_inf()) atomicMin(best_key, f2key(d));
-  }
-  if (st) atomicOr(status, st);
-}
-
-__global__ void k_inside(MeshView m, const double *pts, uint32_t n, Pose16 pose,
-                         sherd_inside_outcome *out, uint32_t *status) {
-  uint32_t st = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double x, y, z;
-    apply_pose(pose.m, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], x, y, z);
-    F3 p = {float(x), float(y), float(z)};
-    sherd_inside_outcome o = {0.0f, 0u};
-    bool in_box = !(p.x < m.lo[0] || p.x > m.hi[0] || p.y < m.lo[1] || p.y > m.hi[1] ||
-                    p.z < m.lo[2] || p.z > m.hi[2]);
-    if (in_box && inside_mesh(m, p, st)) o = {mesh_distance(m, p, f_inf(), st), 1u};
-    out[i] = o;
   }
   if (st) atomicOr(status, st);
 }
@@ -864,6 +870,56 @@ __device__ __forceinline__ bool warp_inside(const MeshView *m, F3 p, bool active
   uint32_t c = 0;
   if (__any_sync(0xffffffffu, third)) c = warp_crossings(m, p, 2, third, par_word);
   return active && (a == b ? a != 0u : c != 0u);
+}
+
+// Inside or not and, inside, the depth. A block takes INSIDE_BLOCK queries at a
+// time: the parities by its warps, then the depths of those inside as walks.
+// Bound by the latency of a block's three steps: 20,000 queries 178 -> 19 us (a
+// thread per query scanning its own cells, then walking while the others of its
+// warp, outside, waited).
+constexpr int INSIDE_BLOCK = 128;
+__global__ void __launch_bounds__(INSIDE_BLOCK) k_inside(const __grid_constant__ MeshView m,
+                                                         const double *pts, uint32_t n,
+                                                         const __grid_constant__ Pose16 pose,
+                                                         sherd_inside_outcome *out, uint32_t *status) {
+  __shared__ unsigned next, found, parity[INSIDE_BLOCK / 32];
+  __shared__ unsigned char queue[INSIDE_BLOCK];
+  __shared__ float4 at[INSIDE_BLOCK];
+  __shared__ WalkSlots<false> slots[INSIDE_BLOCK / 32];
+  const int warp = threadIdx.x >> 5;
+  uint32_t st = 0;
+  for (size_t first = size_t(blockIdx.x) * INSIDE_BLOCK; first < n;
+       first += size_t(gridDim.x) * INSIDE_BLOCK) {
+    if (threadIdx.x == 0) next = found = 0;
+    __syncthreads();
+    const size_t i = first + threadIdx.x;
+    F3 p = {0.0f, 0.0f, 0.0f};
+    bool in_box = false;
+    if (i < n) {
+      double x, y, z;
+      apply_pose(pose.m, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], x, y, z);
+      p = {float(x), float(y), float(z)};
+      in_box = !(p.x < m.lo[0] || p.x > m.hi[0] || p.y < m.lo[1] || p.y > m.hi[1] ||
+                 p.z < m.lo[2] || p.z > m.hi[2]);
+    }
+    const bool inside = warp_inside(&m, p, in_box, parity + warp);
+    if (inside) {
+      at[threadIdx.x] = make_float4(p.x, p.y, p.z, 0.0f);
+      queue[atomicAdd(&found, 1u)] = (unsigned char)threadIdx.x;
+    } else if (i < n) {
+      out[i] = {0.0f, 0u};
+    }
+    __syncthreads();
+    face_walks<false, false>(
+        &next, found, slots[warp],
+        [&](uint32_t k, FaceWalk &w) {
+          const float4 q = at[queue[k]];
+          return walk_start<false>(w, &m, {q.x, q.y, q.z}, f_inf());
+        },
+        [&](uint32_t k, const FaceWalk &w) { out[first + queue[k]] = {w.best, 1u}; }, st);
+    __syncthreads();
+  }
+  if (st) atomicOr(status, st);
 }
 
 __global__ void k_pen_init(PenState ps) {

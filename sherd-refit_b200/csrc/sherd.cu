@@ -966,8 +966,8 @@ int sherd_bounded_distance(sherd_ctx *ctx, const sherd_mesh *mesh, const double 
   if ((rc = upload(ctx, p, points, size_t(3) * n))) return rc;
   if (reduce == SHERD_REDUCE_ALL) {
     CK(o.alloc(n));
-    k_bounded_all<<<blocks_for(n, 128), 128, 0, ctx->stream>>>(mesh->view, p.p, n, pose_of(pose),
-                                                              window, o.p, ctx->d_status);
+    k_bounded_all<<<std::min(blocks_for(n, 128), unsigned(ctx->sm_count) * 16u), 128, 0,
+                    ctx->stream>>>(mesh->view, p.p, n, pose_of(pose), window, o.p, ctx->d_status);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, o.p, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
     return finish(ctx, "bounded_distance", n, true);
@@ -1008,8 +1008,8 @@ int sherd_inside(sherd_ctx *ctx, const sherd_mesh *mesh, const double *points, u
   DBuf<sherd_inside_outcome> o;
   if ((rc = upload(ctx, p, points, size_t(3) * n))) return rc;
   CK(o.alloc(n));
-  k_inside<<<blocks_for(n, 128), 128, 0, ctx->stream>>>(mesh->view, p.p, n, pose_of(pose), o.p,
-                                                       ctx->d_status);
+  k_inside<<<blocks_for(n, INSIDE_BLOCK), INSIDE_BLOCK, 0, ctx->stream>>>(
+      mesh->view, p.p, n, pose_of(pose), o.p, ctx->d_status);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(out, o.p, sizeof(sherd_inside_outcome) * n, cudaMemcpyDeviceToHost,
                      ctx->stream));
