@@ -29,7 +29,7 @@ __device__ __forceinline__ uint32_t block_share(uint32_t n, uint32_t &first) {
   return min(per, n - first);
 }
 
-// Bound by the latency of the walks: a lane's faces shared by its warp, 25,000
+// Bound by the latency of the walks: a lane's faces shared by its warp, 150,000
 // queries 136 -> 66 us (a thread per query with its own loop over a leaf's faces).
 __global__ void __launch_bounds__(128) k_bounded_all(const __grid_constant__ MeshView m,
                                                      const double *pts, uint32_t n,

@@ -31,24 +31,27 @@ __global__ void k_incidence(const uint32_t *f, uint32_t n_corners, uint32_t *ver
   face[i] = i / 3u;
 }
 
-// One thread per vertex over the incidence sorted (stably) by vertex, so its
-// faces come in ascending order, as the reference's face loop adds them; a
-// face that names the vertex twice adds its normal twice, as there.
+// Where each vertex's corners begin in the incidence sorted by vertex; a vertex
+// without any keeps the MISS that `start` was filled with.
+__global__ void k_corner_starts(const uint32_t *vertex, uint32_t n_corners, uint32_t *start) {
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n_corners && (i == 0 || vertex[i] != vertex[i - 1])) start[vertex[i]] = i;
+}
+
+// One thread per vertex (the n of `sel`, or [0, n) without) over the incidence
+// sorted (stably) by vertex, so its faces come in ascending order, as the
+// reference's face loop adds them; a face that names the vertex twice adds its
+// normal twice, as there. Bound by the latency of its dependent loads: a table
+// of the starts took the place of a binary search of 22 of them.
 __global__ void k_vertex_normals(const double *v, const uint32_t *f, const uint32_t *vertex,
-                                 const uint32_t *face, uint32_t n_corners, uint32_t nv,
-                                 double *out) {
-  uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nv) return;
-  uint32_t lo = 0, hi = n_corners;
-  while (lo < hi) {
-    uint32_t mid = lo + (hi - lo) / 2u;
-    if (vertex[mid] < j)
-      lo = mid + 1u;
-    else
-      hi = mid;
-  }
+                                 const uint32_t *face, const uint32_t *start, uint32_t n_corners,
+                                 const uint32_t *sel, uint32_t n_out, double *out) {
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_out) return;
+  const uint32_t j = sel ? sel[i] : i;
   double s[3] = {0.0, 0.0, 0.0};
-  for (uint32_t k = lo; k < n_corners && vertex[k] == j; ++k) {
+  // (MISS is beyond every corner.)
+  for (uint32_t k = start[j]; k < n_corners && vertex[k] == j; ++k) {
     const uint32_t *tri = f + 3 * size_t(face[k]);
     const double *o = v + 3 * size_t(tri[0]), *b = v + 3 * size_t(tri[1]),
                  *c = v + 3 * size_t(tri[2]);
@@ -59,7 +62,7 @@ __global__ void k_vertex_normals(const double *v, const uint32_t *f, const uint3
     s[2] += e1[0] * e2[1] - e1[1] * e2[0];
   }
   double len = sqrt((s[0] * s[0] + s[1] * s[1]) + s[2] * s[2]);
-  double *n = out + 3 * size_t(j);
+  double *n = out + 3 * size_t(i);
   if (len > 0.0) {
     n[0] = s[0] / len;
     n[1] = s[1] / len;
@@ -81,19 +84,6 @@ __global__ void k_fracture_flags(const uint32_t *near, const uint8_t *fracture, 
   uint32_t j = near[i];
   flags[i] = (j != MISS && fracture[j]) ? 1 : 0;
   lin[i] = i;
-}
-
-// refine::cloud_from_indices (refine.rs:208-214): the selected vertices'
-// points and normals, in selection order.
-__global__ void k_gather_cloud(const double *v, const double *normals, const uint32_t *sel,
-                               uint32_t m, double *points_out, double *normals_out) {
-  uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m) return;
-  size_t i = sel[k];
-  for (int a = 0; a < 3; ++a) {
-    points_out[3 * size_t(k) + a] = v[3 * i + a];
-    normals_out[3 * size_t(k) + a] = normals[3 * i + a];
-  }
 }
 
 // ---- placement (types.rs:202-214) ---------------------------------------------

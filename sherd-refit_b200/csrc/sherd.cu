@@ -2351,12 +2351,15 @@ bool all_finite(const double *p, size_t n);
 // refine::vertex_normals (refine.rs:121-151) of a mesh already on the device:
 // the corners sorted stably by vertex, so each vertex adds its faces'
 // unnormalised normals in ascending face order, as the reference's loop does.
+// Of the n vertices of `sel`, in its order, or of all of them (null).
 int vertex_normals_dev(sherd_ctx *ctx, const double *dv, uint32_t nv, const uint32_t *df,
-                       uint32_t nf, DBuf<double> &dn) {
+                       uint32_t nf, const uint32_t *sel, uint32_t n, DBuf<double> &dn) {
   cudaStream_t s = ctx->stream;
   const uint32_t nc = 3u * nf;
-  DBuf<uint32_t> key, key2, face, face2;
-  CK(dn.alloc(size_t(3) * nv));
+  DBuf<uint32_t> key, key2, face, face2, start;
+  CK(dn.alloc(size_t(3) * n));
+  CK(start.alloc(nv));
+  CK(cudaMemsetAsync(start.p, 0xff, sizeof(uint32_t) * nv, s));
   if (nc) {
     CK(key.alloc(nc));
     CK(key2.alloc(nc));
@@ -2368,8 +2371,10 @@ int vertex_normals_dev(sherd_ctx *ctx, const double *dv, uint32_t nv, const uint
     // LSD radix sort is stable: each vertex keeps its faces in ascending order.
     int rc = radix_sort_pairs(ctx, key.p, key2.p, face.p, face2.p, nc, bits);
     if (rc) return rc;
+    k_corner_starts<<<blocks_for(nc), 256, 0, s>>>(key2.p, nc, start.p);
+    CK(cudaGetLastError());
   }
-  k_vertex_normals<<<blocks_for(nv), 256, 0, s>>>(dv, df, key2.p, face2.p, nc, nv, dn.p);
+  k_vertex_normals<<<blocks_for(n), 256, 0, s>>>(dv, df, key2.p, face2.p, start.p, nc, sel, n, dn.p);
   CK(cudaGetLastError());
   return SHERD_OK;
 }
@@ -2607,7 +2612,7 @@ int sherd_vertex_normals(sherd_ctx *ctx, const double *v, uint32_t nv, const uin
       (rc = chk.read(ctx, &got)))
     return rc;
   if (got.bad_index) return fail(ctx, SHERD_E_INVALID, "face index beyond the vertex array");
-  if ((rc = vertex_normals_dev(ctx, dv.p, nv, df.p, nf, dn))) return rc;
+  if ((rc = vertex_normals_dev(ctx, dv.p, nv, df.p, nf, nullptr, nv, dn))) return rc;
   CK(cudaMemcpyAsync(normals, dn.p, 24 * size_t(nv), cudaMemcpyDeviceToHost, ctx->stream));
   return finish(ctx, "vertex_normals", nv, true);
 }
@@ -2666,23 +2671,22 @@ int sherd_fracture_cloud(sherd_ctx *ctx, const double *v, uint32_t nv, const uin
   DBuf<unsigned char> tmp;
   CK(tmp.alloc(bytes));
   CK(cub::DeviceSelect::Flagged(tmp.p, bytes, lin.p, flags.p, sel.p, nsel.p, int(nv), s));
-  // Every vertex's normal (refine.rs:121-151), then the selected vertices'
-  // points and normals gathered in selection order.
-  if ((rc = vertex_normals_dev(ctx, dv.p, nv, df.p, nf, dn))) return rc;
   uint32_t count = 0;
   CK(cudaMemcpyAsync(&count, nsel.p, 4, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   *n_out = count;
   const uint32_t m = std::min(count, cap);
   if (m) {
-    DBuf<double> gp, gn;
+    // The selected vertices' normals (refine.rs:121-151) and points
+    // (cloud_from_indices, refine.rs:208-214), in selection order.
+    DBuf<double> gp;
+    if ((rc = vertex_normals_dev(ctx, dv.p, nv, df.p, nf, sel.p, m, dn))) return rc;
     CK(gp.alloc(size_t(3) * m));
-    CK(gn.alloc(size_t(3) * m));
-    k_gather_cloud<<<blocks_for(m), 256, 0, s>>>(dv.p, dn.p, sel.p, m, gp.p, gn.p);
+    k_gather_points<<<blocks_for(m), 256, 0, s>>>(dv.p, sel.p, m, gp.p);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(idx_out, sel.p, 4 * size_t(m), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(points_out, gp.p, 24 * size_t(m), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(normals_out, gn.p, 24 * size_t(m), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(normals_out, dn.p, 24 * size_t(m), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
   }
   return finish(ctx, "fracture_cloud", nv, true);
