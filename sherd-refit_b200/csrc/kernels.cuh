@@ -938,6 +938,8 @@ __global__ void __launch_bounds__(256, PEN_INSIDE_MINB) k_pen_inside(const PairV
                                                     unsigned long long budget, uint32_t *status) {
   __shared__ WarpQueue wqs[8];
   __shared__ unsigned parity[8];
+  __shared__ WalkSlots<false> walk_slots[8];
+  WalkSlots<false> &slots = walk_slots[threadIdx.x >> 5];
   WarpQueue &q = wqs[threadIdx.x >> 5];
   unsigned *par_word = parity + (threadIdx.x >> 5);
   int lane = threadIdx.x & 31;
@@ -956,29 +958,35 @@ __global__ void __launch_bounds__(256, PEN_INSIDE_MINB) k_pen_inside(const PairV
   // of inside points, so the last point to raise it holds the true maximum.
   auto depth_stage = [&](bool drain) {
     while (q.n_in >= 32 || (drain && q.n_in > 0)) {
-      unsigned long long e;
-      if (wq_pop(q.in, &q.n_in, e)) {
-        uint32_t u = uint32_t(e >> 32), i = uint32_t(e);
+      unsigned long long e = 0;
+      const bool got = wq_pop(q.in, &q.n_in, e);
+      const uint32_t u = uint32_t(e >> 32);
+      const MeshView *m = nullptr;
+      F3 p = {0.0f, 0.0f, 0.0f};
+      float w = 0.0f, top = 0.0f;
+      if (got) {
         PenUnit x = pen_unit(pairs, items, cands, inv, u);
-        const MeshView &m = *x.mesh;
-        F3 p = unit_point(x, i);
-        const float w = __double2float_rd(x.pen);
-        const bool deeper = !(mesh_may_reach(m, p, w) && mesh_any_within(m, p, w, st));
+        m = x.mesh;
+        p = unit_point(x, uint32_t(e));
+        w = __double2float_rd(x.pen);
+      }
+      const bool deeper =
+          warp_walks<true>(m, p, w, got && mesh_may_reach(*m, p, w), slots, st) == f_inf();
+      bool raise = got, look = false;
+      if (got) {
         if (deeper) atomicAdd(&ps.deeper[u], 1u);
         const unsigned key = *((volatile unsigned *)&ps.deep[u]);
-        bool raise = true;
         if (key != 0u) {
-          const float top = key2f(key - 1u);
+          top = key2f(key - 1u);
           if (!deeper && top >= w)
             raise = false;  // D <= w <= M
-          else if (mesh_may_reach(m, p, top) && mesh_any_within(m, p, top, st))
-            raise = false;  // D <= M
-        }
-        if (raise) {
-          float depth = mesh_distance(m, p, deeper ? f_inf() : w, st);
-          atomicMax(&ps.deep[u], f2key(depth) + 1u);
+          else
+            look = mesh_may_reach(*m, p, top);
         }
       }
+      if (warp_walks<true>(m, p, top, look, slots, st) != f_inf()) raise = false;  // D <= M
+      const float depth = warp_walks<false>(m, p, deeper ? f_inf() : w, raise, slots, st);
+      if (raise) atomicMax(&ps.deep[u], f2key(depth) + 1u);
     }
   };
   auto parity_stage = [&](bool drain) {
