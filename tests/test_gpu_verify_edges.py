@@ -75,3 +75,16 @@ def test_candidates_do_not_depend_on_the_batch_size(sherd, gpu_ctx, gpu_slab, sl
         got[n] = sherd.candidates(gpu_ctx.ladder_verify_batch([gpu_slab["pair"]], items, params)).copy()
     for n in sizes:
         assert got[n].tobytes() == got[sizes[-1]][:n].tobytes(), n
+
+
+@pytest.mark.parametrize("far", [3e4, 3e6, 4e7, 5e17])
+def test_scores_of_runaway_poses_are_the_oracles(gpu_ctx, gpu_slab, oracle, slab, far):
+    """Poses at which f32 merges points, and then faces: the least distance is still exact."""
+    scales = oracle.scales_from(slab["scales"])
+    g, c = ([_side(lib, MESHES["ball"](), np.random.default_rng(i), 500, 2000, 70) for i in (1, 2)]
+            for lib in (gpu_ctx, oracle))
+    pose = _pose(0.4, [far, -0.3 * far, 0.1 * far])
+    sg = gpu_ctx.verify(g[0], g[1], pose, gpu_slab["scales"])
+    sc = oracle.verify(c[0], c[1], pose, scales)
+    for key in SCORE_KEYS:
+        assert np.array_equal(getattr(sg, key), getattr(sc, key), equal_nan=True), key
