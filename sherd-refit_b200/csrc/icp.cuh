@@ -1036,6 +1036,9 @@ __device__ __forceinline__ void icp_pass(const double4 *src, uint32_t ns, const 
     if (threadIdx.x < ICP_BLOCK)
       p2p_accumulate<false, C>(src, ns, tgt, sh.t, r2, valid, m.hint, mean, one_over_n, sh);
     reduce_sums(sh, 8, 17);
+    // Every CTA has read every match: only now may one of them write the next
+    // pass's (the point-to-plane sums have this barrier before their exchange).
+    if constexpr (C > 1) rung_sync<C>();
     return;
   }
   icp_sums<G, C>(src, ns, tgt, r2, valid, b, m);

@@ -61,6 +61,22 @@ def test_a_start_is_registered_alike_in_every_form(gpu_ctx, oracle, n, estimatio
             assert int(g["correspondences"]) == r.correspondences
 
 
+@pytest.mark.parametrize("estimation", [1, 0], ids=["plane", "point"])
+@pytest.mark.parametrize("n", [20_011, 200_001])
+def test_large_sources_are_registered_alike_in_every_form(gpu_ctx, n, estimation):
+    """Long passes, in which the blocks of a cluster drift apart: none may write its matches while
+    another still sums over them."""
+    rng = np.random.default_rng(n)
+    tp, tn = _surface(rng, 3000)
+    src, _ = _surface(rng, n)
+    target = gpu_ctx.cloud(tp, tn)
+    starts = _starts(rng, 297)
+    whole = gpu_ctx.icp_rung_array(src, target, starts, 0.2 * T, 12, estimation=estimation)
+    for k in (1, 18, 37, 74) * 3:
+        some = gpu_ctx.icp_rung_array(src, target, starts[:k], 0.2 * T, 12, estimation=estimation)
+        assert some.tobytes() == whole[:k].tobytes(), k
+
+
 @pytest.mark.parametrize("distance", [1e-3, 0.5, 40.0, 1e4])
 def test_radii_from_no_match_to_every_point(gpu_ctx, oracle, distance):
     rng = np.random.default_rng(5)
