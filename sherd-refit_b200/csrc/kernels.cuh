@@ -472,6 +472,8 @@ __global__ void __launch_bounds__(ICP_BLOCK *G, MINB) k_ladder(const PairView *p
   const IcpMemory<H> mine = memory_slot(mem, blockIdx.x / C, stride);
   unsigned long long start = global_ns();
   unsigned it;
+  // A CTA's shared memory may be written by another once it is known to run.
+  if constexpr (C > 1) rung_sync<C>();
   while (take_shared<C>(q, start, it, st)) {
     const sherd_work_item &w = items[it];
     const PairView &pr = pairs[w.pair];

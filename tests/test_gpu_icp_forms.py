@@ -117,3 +117,27 @@ def test_targets_above_16_bits_and_batches_of_every_form(sherd, gpu_ctx, gpu_sla
         plain = sherd.candidates(gpu_ctx.ladder_verify_batch([pair], items[:40],
                                                              sherd.default_params(), sherd.SCHED_PLAIN))
         assert plain.tobytes() == cands[:40].tobytes()
+
+
+@pytest.mark.parametrize("limit", [0.0, 0.3], ids=["plain_ladder", "early_rejection"])
+@pytest.mark.parametrize("n", [300, 600, 1100, 2100])
+def test_ladders_run_alike_in_every_form(sherd, gpu_ctx, gpu_slab, slab, n, limit):
+    """The queue's items shared by a cluster's blocks, in one launch or split by the early
+    rejection: the same candidates on clusters of 8, 4 and 2 blocks, on wide blocks and on narrow
+    ones, under both schedules."""
+    rng = np.random.default_rng(n)
+    tp, tn = _surface(rng, 3000)
+    src, _ = _surface(rng, n)
+    pair = gpu_ctx.pair(gpu_slab["a"]["surf"], gpu_slab["b"]["surf"], gpu_ctx.cloud(tp, tn),
+                        gpu_slab["frac_t"], src, src[:n // 2], gpu_slab["scales"])
+    inits = np.concatenate([slab["starts"].reshape(-1, 4, 4), _starts(rng, 20)])
+    params = sherd.default_params()
+    params.early_reject_tight = limit
+
+    def run(k, sched):
+        items = [(0, i, inits[i % len(inits)]) for i in range(k)]
+        return sherd.candidates(gpu_ctx.ladder_verify_batch([pair], items, params, sched)).copy()
+    whole = run(max(STARTS), sherd.SCHED_BATCHED)
+    for k in STARTS * 2:
+        for sched in (sherd.SCHED_BATCHED, sherd.SCHED_PLAIN):
+            assert run(k, sched).tobytes() == whole[:k].tobytes(), (k, sched)
