@@ -1964,7 +1964,13 @@ int batch_create(sherd_ctx *ctx, const std::vector<PairView> &views, const sherd
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_v, k_verify_items, VER_BLOCK, 0));
   b->grid_l = unsigned(std::max(1, b->occ[LADDER_DEFAULT]) * ctx->sm_count);
   b->grid_v = unsigned(std::max(1, occ_v) * ctx->sm_count);
-  CK(b->scratch.alloc(size_t(b->grid_v) * b->max_scratch));
+  // Scratch for the blocks that a verification is launched with: its items at a time
+  // (a pair's under the plain schedule), or four an item side by side.
+  uint32_t most = sched == SHERD_SCHED_BATCHED ? n_items : 0;
+  for (uint32_t c : b->pair_count) most = std::max(most, c);
+  uint32_t blocks_v = std::min(most, b->grid_v);
+  if (sched == SHERD_SCHED_BATCHED && !b->early() && verify_in_parts(b, n_items)) blocks_v = 4 * n_items;
+  CK(b->scratch.alloc(size_t(std::max(1u, blocks_v)) * b->max_scratch));
   if (sched == SHERD_SCHED_BATCHED) {
     // Unit 2i is item i's side 0 (B's samples in A's mesh), 2i+1 its side 1.
     std::vector<uint32_t> chunk0(2 * size_t(n_items) + 1);
@@ -2003,9 +2009,9 @@ int batch_create(sherd_ctx *ctx, const std::vector<PairView> &views, const sherd
     b->grid_m = unsigned(std::max(1, occ_m) * ctx->sm_count);
   }
   b->hint_stride = (b->hint_stride + 63) / 64 * 64;
-  // The plain schedule launches one block or cluster per item of a pair, so it
-  // needs as many hint slots as the largest pair has items.
-  size_t slots = std::max<size_t>(b->grid_l, 2 * size_t(ctx->sm_count));
+  // A slot for every item in flight: the plain schedule launches one block or
+  // cluster per item of a pair, early rejection up to grid_l of them.
+  size_t slots = b->early() ? std::min<size_t>(b->grid_l, n_items) : 0;
   for (uint32_t c : b->pair_count) slots = std::max<size_t>(slots, c);
   if (sched == SHERD_SCHED_BATCHED) {
     // The buckets' launches run side by side, each on its own slice of slots,

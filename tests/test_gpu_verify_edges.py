@@ -88,3 +88,34 @@ def test_scores_of_runaway_poses_are_the_oracles(gpu_ctx, gpu_slab, oracle, slab
     sc = oracle.verify(c[0], c[1], pose, scales)
     for key in SCORE_KEYS:
         assert np.array_equal(getattr(sg, key), getattr(sc, key), equal_nan=True), key
+
+
+def test_one_pose_holds_scratch_for_one_pose(sherd, gpu_slab, slab):
+    """Device memory goes by the items of a call, not by what the device could run at once: at
+    10^6 samples a side one item takes four score blocks' scratch of 4 MB each (444 blocks' would
+    be 1.8 GB), and a ladder of two items two slots of 200,000 points (592 slots' would be 1 GB).
+    """
+    import torch
+
+    ctx = sherd.Context(0)
+    n = 1_000_000
+    a, b = (_side(ctx, MESHES["ball"](), np.random.default_rng(i), n, 5000, 70) for i in (1, 2))
+    rng = np.random.default_rng(3)
+    src = rng.normal(size=(200_000, 3))
+    tgt = rng.normal(size=(500, 3))
+    cloud = ctx.cloud(tgt, tgt / np.linalg.norm(tgt, axis=1, keepdims=True))
+    pair = ctx.pair(a, b, cloud, cloud, src, src, gpu_slab["scales"])
+    pose = _pose(0.3, [0.1, 0.2, 0.3])
+
+    def held(call):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        call()
+        return before - torch.cuda.mem_get_info()[0]
+    assert held(lambda: ctx.verify(a, b, pose, gpu_slab["scales"])) < 200 << 20
+    items = [(0, k, pose) for k in range(2)]
+    for sched in (sherd.SCHED_BATCHED, sherd.SCHED_PLAIN):
+        for limit in (0.0, 0.3):
+            params = sherd.default_params()
+            params.early_reject_tight = limit
+            assert held(lambda: ctx.ladder_verify_batch([pair], items, params, sched)) < 200 << 20
