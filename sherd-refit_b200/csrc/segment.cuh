@@ -113,10 +113,16 @@ constexpr int BALL_WARPS = 4;
 constexpr int BALL_BLOCK = 512;
 constexpr uint32_t BALL_BLOCK_STACK = 2048;
 
+// Entries kept free for going down one node at a time, which adds one a level: a
+// Karras tree's path takes each of the 63 code bits, and where codes are equal
+// each of the 32 index bits, at most once.
+constexpr int BALL_RESERVE = 63 + 32 + 1;
+
 // Nodes to take at a time: each may put two back, and from one at a time on the
 // stack grows by no more than the tree's depth.
-__device__ __forceinline__ int ball_width(int sp, uint32_t stack, int most) {
-  return min(sp, max(1, min(most, int(stack) - 80 - sp)));
+__host__ __device__ __forceinline__ int ball_width(int sp, uint32_t stack, int most) {
+  const int room = int(stack) - BALL_RESERVE - sp, width = room < most ? room : most;
+  return width < 1 ? 1 : width < sp ? width : sp;
 }
 
 struct BallSums {
@@ -196,7 +202,7 @@ struct BallWarp {
 
 __global__ void __launch_bounds__(BALL_WARPS * 32)
     k_ball_warp(CloudView all, const double *cent, const uint32_t *rep, uint32_t n_rep,
-                double radius, BallSums w, uint32_t *large, uint32_t *n_large) {
+                double radius, BallSums w, uint32_t *large, uint32_t *n_large, uint32_t *status) {
   const unsigned FULL = 0xffffffffu;
   __shared__ BallWarp mem[BALL_WARPS];
   BallWarp &b = mem[threadIdx.x >> 5];
@@ -205,6 +211,7 @@ __global__ void __launch_bounds__(BALL_WARPS * 32)
   const double r2 = radius * radius;
   const float bound = ball_bound(all, radius), b2 = bound * bound;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  uint32_t st = 0;
   for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_rep; r += warps) {
     const double *c0 = cent + 3 * size_t(rep[r]);
     const double q[3] = {c0[0], c0[1], c0[2]};
@@ -237,8 +244,13 @@ __global__ void __launch_bounds__(BALL_WARPS * 32)
       for (int c = 0; c < 2; ++c) {
         for (int k = 0; __any_sync(FULL, cnt[c] > k); ++k) take(cnt[c] > k, ref[c] + k);
         const unsigned open = __ballot_sync(FULL, cnt[c] == 0);
-        if (cnt[c] == 0) b.stack[sp + __popc(open & below)] = ref[c];
+        const int at = sp + __popc(open & below);
+        if (cnt[c] == 0 && at < int(BALL_STACK)) b.stack[at] = ref[c];
         sp += __popc(open);
+        if (sp > int(BALL_STACK)) {  // the same for the warp
+          st |= ST_STACK;
+          sp = int(BALL_STACK);
+        }
       }
       __syncwarp();
     }
@@ -275,6 +287,7 @@ __global__ void __launch_bounds__(BALL_WARPS * 32)
     if (lane == 0) ball_result(w, r, n, b.sum);
     __syncwarp();
   }
+  if (st && lane == 0) atomicOr(status, st);
 }
 
 // The listed representatives, a block each; `cap` (a power of two) member slots in
@@ -283,7 +296,7 @@ __global__ void __launch_bounds__(BALL_WARPS * 32)
 __global__ void __launch_bounds__(BALL_BLOCK)
     k_ball_block(CloudView all, const double *cent, const uint32_t *rep, const uint32_t *list,
                  uint32_t n_list, double radius, BallSums w, uint32_t cap, uint32_t *max_members,
-                 uint32_t *max_ranges) {
+                 uint32_t *max_ranges, uint32_t *status) {
   extern __shared__ __align__(16) unsigned char ball_dynamic[];
   double *part = reinterpret_cast<double *>(ball_dynamic);               // 4 x BALL_BLOCK
   int *stack = reinterpret_cast<int *>(part + 4 * BALL_BLOCK);           // BALL_BLOCK_STACK
@@ -291,6 +304,7 @@ __global__ void __launch_bounds__(BALL_BLOCK)
   __shared__ uint32_t s_n, s_sp, s_ranges;
   __shared__ double s_sum[4];
   const uint32_t tid = threadIdx.x;
+  uint32_t st = 0;
   const double r2 = radius * radius;
   const float bound = ball_bound(all, radius), b2 = bound * bound;
   for (uint32_t e = blockIdx.x; e < n_list; e += gridDim.x) {
@@ -318,7 +332,7 @@ __global__ void __launch_bounds__(BALL_BLOCK)
       take(0, int(all.root_leaf));
     }
     for (;;) {
-      const int sp = int(s_sp);
+      const int sp = int(min(s_sp, BALL_BLOCK_STACK));
       if (sp == 0) break;
       const int width = ball_width(sp, BALL_BLOCK_STACK, BALL_BLOCK);
       const bool mine = int(tid) < width;
@@ -334,7 +348,11 @@ __global__ void __launch_bounds__(BALL_BLOCK)
             atomicAdd(&s_ranges, 1u);
             take(ref[c], cnt[c]);
           } else if (cnt[c] == 0) {
-            stack[atomicAdd(&s_sp, 1u)] = ref[c];
+            const uint32_t at = atomicAdd(&s_sp, 1u);
+            if (at < BALL_BLOCK_STACK)
+              stack[at] = ref[c];
+            else
+              st |= ST_STACK;
           }
         }
       }
@@ -376,6 +394,7 @@ __global__ void __launch_bounds__(BALL_BLOCK)
     }
     __syncthreads();
   }
+  if (st) atomicOr(status, st);
 }
 
 // A representative's answer to every face it represents.

@@ -2320,7 +2320,7 @@ int ball_pass(sherd_ctx *ctx, const CloudView &all, const double *cent, const ui
   CK(cudaMemsetAsync(mx.p, 0, 12, s));
   k_ball_warp<<<std::max(1u, std::min(blocks_for(size_t(n_rep) * 32, BALL_WARPS * 32),
                                       unsigned(ctx->sm_count) * 32u)),
-                BALL_WARPS * 32, 0, s>>>(all, cent, rep, n_rep, radius, sums, large.p, mx.p);
+                BALL_WARPS * 32, 0, s>>>(all, cent, rep, n_rep, radius, sums, large.p, mx.p, ctx->d_status);
   CK(cudaGetLastError());
   uint32_t h[3] = {};
   CK(cudaMemcpyAsync(h, mx.p, 4, cudaMemcpyDeviceToHost, s));
@@ -2329,7 +2329,7 @@ int ball_pass(sherd_ctx *ctx, const CloudView &all, const double *cent, const ui
     const size_t bytes = size_t(32) * BALL_BLOCK + size_t(4) * BALL_BLOCK_STACK + size_t(4) * cap;
     CK(cudaFuncSetAttribute(k_ball_block, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
     k_ball_block<<<std::min(h[0], unsigned(ctx->sm_count) * 4u), BALL_BLOCK, bytes, s>>>(
-        all, cent, rep, large.p, h[0], radius, sums, cap, mx.p + 1, mx.p + 2);
+        all, cent, rep, large.p, h[0], radius, sums, cap, mx.p + 1, mx.p + 2, ctx->d_status);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(h + 1, mx.p + 1, 8, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
