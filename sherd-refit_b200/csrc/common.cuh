@@ -29,10 +29,6 @@ constexpr int POINT_LEAF = POINT_LEAF_MAX;  // points per BVH leaf, at most
 #ifndef PEN_INSIDE_MINB
 #define PEN_INSIDE_MINB 4
 #endif
-// Whether point clouds carry the 4-wide tree that nearest_within_sq walks.
-#ifndef WIDE_NN
-#define WIDE_NN 1
-#endif
 constexpr int STACK = 64;      // traversal stack entries (Karras depth <= 63 + log2 n)
 
 __host__ __device__ inline float f_inf() { return __builtin_huge_valf(); }

@@ -81,7 +81,7 @@ struct CloudView {
   uint32_t n;
   uint32_t root_leaf;
   float pad;
-  const WNode *wide;   // the 4-wide form of `nodes`, or null
+  const WNode *wide;   // the 4-wide form of `nodes` (null with root_leaf)
 };
 
 // ---- Morton codes -----------------------------------------------------------

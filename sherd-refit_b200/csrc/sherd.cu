@@ -572,7 +572,7 @@ int cloud_build_dev(sherd_ctx *ctx, const double *dp, const double *dn, uint32_t
                                                        dn ? c->nrm.p : nullptr);
   CK(cudaGetLastError());
   const bool tree = np > uint32_t(POINT_LEAF);
-  if (tree && WIDE_NN) {
+  if (tree) {
     CK(c->wide.alloc(np - 1));
     k_widen<<<blocks_for(np - 1), 256, 0, ctx->stream>>>(c->nodes.p, int(np - 1), c->wide.p);
     CK(cudaGetLastError());
@@ -585,7 +585,7 @@ int cloud_build_dev(sherd_ctx *ctx, const double *dp, const double *dn, uint32_t
   v.n = np;
   v.root_leaf = np <= uint32_t(POINT_LEAF) ? np : 0;
   v.pad = pad;
-  v.wide = tree && WIDE_NN ? c->wide.p : nullptr;
+  v.wide = c->wide.p;
   return SHERD_OK;
 }
 

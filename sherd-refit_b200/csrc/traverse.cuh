@@ -479,54 +479,8 @@ __device__ __noinline__ int nearest_within_sq(const CloudView &c, double qx, dou
   }
   // Box distances are taken from the f32-rounded query; the padding of the
   // boxes (>= the rounding of the query) keeps them lower bounds.
-  int stack_n[STACK];
-  float stack_k[STACK];
-  int sp = 0, node = 0;
-  uint32_t visits = 0;
-  if (c.wide) {
-    wide_walk(
-        c.wide, qc, 2u * c.n + 64u,
-        leaf, bound2, [](float) {}, status);
-    return best_s;
-  }
-  for (;;) {
-    if (++visits > 2u * c.n + 64u) {
-      status |= ST_STACK;
-      break;
-    }
-    Child2 n = load_node(c.nodes, node);
-    float k[2] = {box_dist2(n.lo0, n.hi0, qc), box_dist2(n.lo1, n.hi1, qc)};
-    int near_c = k[1] < k[0] ? 1 : 0;
-    int next = -1;
-    for (int q = 0; q < 2; ++q) {
-      int ch = q == 0 ? near_c : 1 - near_c;
-      if (!(k[ch] <= bound2())) continue;
-      if (n.cnt[ch]) {
-        leaf(n.ref[ch], n.cnt[ch]);
-      } else if (next < 0) {
-        next = n.ref[ch];
-      } else if (sp < STACK) {
-        stack_n[sp] = n.ref[ch];
-        stack_k[sp++] = k[ch];
-      } else {
-        status |= ST_STACK;
-      }
-    }
-    if (next >= 0) {
-      node = next;
-      continue;
-    }
-    bool more = false;
-    while (sp > 0) {
-      --sp;
-      if (stack_k[sp] <= bound2()) {
-        node = stack_n[sp];
-        more = true;
-        break;
-      }
-    }
-    if (!more) break;
-  }
+  wide_walk(
+      c.wide, qc, 2u * c.n + 64u, leaf, bound2, [](float) {}, status);
   return best_s;
 }
 

@@ -115,3 +115,13 @@ def test_samples_without_a_breakline_have_no_margin(sherd, oracle, slab):
     md = pre.match_data(_Device(oracle), p["V"], p["F"], np.ones(len(p["F"]), bool), 30.0, 0)
     assert len(md.brk) == 0 and len(md.samples.margin_idx) == 0
     assert len(md.samples.pf) == 12000      # every face is fracture: the count hits the cap
+
+
+def test_every_build_switch_is_one_a_build_may_change():
+    """The kernels' compile-time switches are sizes and limits; none turns off a structure that a
+    kernel walks without asking for it."""
+    import re
+    from pathlib import Path
+    csrc = Path(__file__).resolve().parent.parent / "sherd-refit_b200" / "csrc"
+    switches = {m for p in csrc.glob("*.cu*") for m in re.findall(r"^#ifndef (\w+)", p.read_text(), re.M)}
+    assert switches <= {"TRI_LEAF_MAX", "POINT_LEAF_MAX", "PEN_INSIDE_MINB", "MIN_REFILL", "MIN_LOOK"}
