@@ -550,9 +550,14 @@ __global__ void __launch_bounds__(PART_BLOCK) k_verify_parts(const PairView *pai
                                                              unsigned *scratch, size_t stride,
                                                              sherd_candidate *out, int full,
                                                              double *inv, int pose_rung,
-                                                             uint32_t *status) {
+                                                             StopCtl stop, uint32_t *status) {
   __shared__ VerShared sh;
   uint32_t st = 0;
+  // Asked to stop (in the ladder, say): as a queue would, nothing more is begun.
+  if (__syncthreads_or(threadIdx.x == 0 && stop_asked(stop))) {
+    if (threadIdx.x == 0) atomicOr(status, ST_ABORTED);
+    return;
+  }
   const uint32_t it = blockIdx.x >> 2, part = blockIdx.x & 3u;
   const PairView &pr = pairs[items[it].pair];
   sherd_candidate *c = out + it;

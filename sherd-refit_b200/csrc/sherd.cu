@@ -1796,7 +1796,7 @@ int launch_verify(sherd_batch *b, cudaStream_t s, int full) {
   if (!b->early() && verify_in_parts(b, b->n_items)) {
     k_verify_parts<<<4 * b->n_items, PART_BLOCK, 0, s>>>(b->dv.p, b->di.p, b->scratch.p,
                                                          b->max_scratch, b->dc.p, full, b->inv.p, 3,
-                                                         ctx->d_status);
+                                                         b->stop(), ctx->d_status);
     CK(cudaGetLastError());
     k_verify_join<<<blocks_for(b->n_items), 256, 0, s>>>(b->dv.p, b->di.p, b->dc.p, full, b->n_items);
     CK(cudaGetLastError());

@@ -6,6 +6,8 @@ Every score is the oracle's, bit for bit, as in the fixture's verification test.
 
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import pytest
 
@@ -119,3 +121,27 @@ def test_one_pose_holds_scratch_for_one_pose(sherd, gpu_slab, slab):
             params = sherd.default_params()
             params.early_reject_tight = limit
             assert held(lambda: ctx.ladder_verify_batch([pair], items, params, sched)) < 200 << 20
+
+
+def test_an_aborted_ladder_is_not_verified(sherd, gpu_slab):
+    """A batch small enough for its scores to go side by side, aborted while its ladder runs, does
+    not begin them: the verification stage takes next to nothing of its own time."""
+    ctx = sherd.Context(0)
+    n = 500_000
+    a, b = (_side(ctx, MESHES["ball"](), np.random.default_rng(i), n, 500, 70) for i in (1, 2))
+    rng = np.random.default_rng(3)
+    src, tgt = rng.normal(size=(400_000, 3)), rng.normal(size=(5000, 3))
+    cloud = ctx.cloud(tgt, tgt / np.linalg.norm(tgt, axis=1, keepdims=True))
+    pair = ctx.pair(a, b, cloud, cloud, src, src, gpu_slab["scales"])
+    items = [(0, k, _pose(0.01 * k, [0.1, 0.2, 0.3])) for k in range(70)]
+    batch = ctx.batch([pair], items, sherd.default_params())
+    whole = batch.run()
+    assert whole["ladder"] > 100.0  # milliseconds: the abort below comes while it runs
+    stop = threading.Timer(0.02, ctx.abort)
+    ms = np.zeros(len(batch.STAGES), np.float32)
+    stop.start()
+    code = sherd.lib().sherd_batch_run(batch.h, ms)
+    stop.join()
+    assert code == -4
+    assert ms[1] < 0.2 * whole["verify"], (whole, ms)
+    assert batch.run().keys() == whole.keys()
