@@ -310,8 +310,9 @@ int sherd_icp_rung(sherd_ctx *ctx, const double *source, uint32_t n_source,
  * calls share them, so two calls that overlap on the GPU (from two
  * contexts, or two host threads on different contexts of one device) race.
  * The first call on each device looks the arrays' device addresses up
- * (cudaGetSymbolAddress) with that device current; make that first call
- * before any stream capture on the device. */
+ * (cudaGetSymbolAddress) with that device current and loads the rung's kernels,
+ * whose code takes device memory; make that first call up front, and before any
+ * stream capture on the device. */
 #define SHERD_NOALLOC_CAPACITY (1u << 20)
 int sherd_icp_rung_noalloc(sherd_ctx *ctx, const double *source, uint32_t n_source,
                            const sherd_cloud *target, const double *inits, uint32_t k,

@@ -122,6 +122,14 @@ cudaError_t noalloc_address(int device, IcpMemory<int> *out) {
   if (e == cudaSuccess) e = cudaGetSymbolAddress(&s, g_noalloc_slacks);
   if (e == cudaSuccess) e = cudaGetSymbolAddress(&c, g_noalloc_chunks);
   if (e == cudaSuccess) e = cudaGetSymbolAddress(&b, g_noalloc_balls);
+  // Kernels are loaded when they are first asked for, which takes device memory
+  // (2 MB for the second of these forms): all of them now, whichever comes first.
+  const void *const forms[] = {(const void *)k_icp_rung<2, 1>, (const void *)k_icp_rung<4, 1>,
+                               (const void *)k_icp_rung<4, 2>, (const void *)k_icp_rung<4, 4>,
+                               (const void *)k_icp_rung<4, 8>};
+  cudaFuncAttributes attributes;
+  for (const void *f : forms)
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&attributes, f);
   if (e != cudaSuccess) return e;
   *out = {static_cast<int *>(h), static_cast<float *>(s), static_cast<IcpChunk *>(c),
           static_cast<float4 *>(b)};
@@ -1381,8 +1389,8 @@ int sherd_icp_rung_noalloc(sherd_ctx *ctx, const double *source, uint32_t n_sour
   CtxLock lock(ctx);
   int rc = begin(ctx);  // makes the context's device current
   if (rc) return rc;
-  // The first call on a device looks the arrays' addresses up; that call should
-  // come before any stream capture on the device.
+  // The first call on a device looks the arrays' addresses up and loads the kernels;
+  // that call should come before any stream capture on the device.
   IcpMemory<int> mem;
   CK(noalloc_address(ctx->device, &mem));
   if (uint64_t(k) * ((n_source + 31u) / 32u) > NOALLOC_CHUNKS) mem.chunks = nullptr, mem.balls = nullptr;

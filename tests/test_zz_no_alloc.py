@@ -94,3 +94,42 @@ def test_the_allocation_free_rung_refuses_what_it_cannot_hold(sherd, gpu_ctx, sl
     rc = _call(sherd, gpu_ctx, d_src.data_ptr(), n, target, host_inits.ctypes.data, 1, opt,
                d_out.data_ptr())
     assert rc == -1 and b"device" in sherd.lib().sherd_last_error(gpu_ctx.h)
+
+
+FIRST_CALLS = """
+import ctypes as C, sys
+sys.path.insert(0, sys.argv[1])
+from importlib import import_module
+import numpy as np
+import torch
+sherd = import_module("sherd-refit_b200")
+ctx = sherd.Context(0)
+p = np.random.default_rng(0).normal(size=(3000, 3))
+target = ctx.cloud(p, p / np.linalg.norm(p, axis=1, keepdims=True))
+src = torch.zeros((4096, 4), dtype=torch.float64, device="cuda")
+src[:, :3] = torch.from_numpy(np.random.default_rng(1).normal(size=(4096, 3)))
+inits = torch.eye(4, dtype=torch.float64, device="cuda").reshape(1, 16).repeat(400, 1).contiguous()
+out = torch.empty(C.sizeof(sherd.Registration) * 400, dtype=torch.uint8, device="cuda")
+free = []
+# The sizes by which a rung takes its blocks and clusters, on 148 SMs.
+for k, n in ((400, 100), (100, 600), (60, 600), (30, 1100), (10, 4000)):
+    rc = sherd.lib().sherd_icp_rung_noalloc(
+        ctx.h, C.c_void_p(src.data_ptr()), n, target.h, C.c_void_p(inits.data_ptr()), k,
+        sherd.IcpOptions(1, 3, 0.5), C.c_void_p(out.data_ptr()))
+    assert rc == 0, sherd.lib().sherd_last_error(ctx.h)
+    free.append(torch.cuda.mem_get_info()[0])
+print(free)
+assert len(set(free)) == 1, free
+"""
+
+
+def test_after_the_first_call_no_form_of_the_rung_takes_device_memory():
+    """The rung runs on blocks and clusters by its size: a call of one form up front must do for
+    all of them. In a process of its own, in which nothing has been loaded before."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    run = subprocess.run([sys.executable, "-c", FIRST_CALLS, str(Path(__file__).resolve().parent.parent)],
+                         capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stdout + run.stderr
