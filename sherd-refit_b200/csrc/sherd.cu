@@ -2333,9 +2333,17 @@ int ball_pass(sherd_ctx *ctx, const CloudView &all, const double *cent, const ui
   uint32_t h[3] = {};
   CK(cudaMemcpyAsync(h, mx.p, 4, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
-  for (uint32_t cap = 8192; h[0]; cap = 32768) {
-    const size_t bytes = size_t(32) * BALL_BLOCK + size_t(4) * BALL_BLOCK_STACK + size_t(4) * cap;
-    CK(cudaFuncSetAttribute(k_ball_block, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+  constexpr uint32_t CAPS[2] = {8192, 32768};
+  auto shared_bytes = [](uint32_t cap) {
+    return size_t(32) * BALL_BLOCK + size_t(4) * BALL_BLOCK_STACK + size_t(4) * cap;
+  };
+  // The most that is ever asked for: the limit is the kernel's, so a smaller one set
+  // here could come between another thread's setting and its launch.
+  if (h[0])
+    CK(cudaFuncSetAttribute(k_ball_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            int(shared_bytes(CAPS[1]))));
+  for (uint32_t cap = CAPS[0]; h[0]; cap = CAPS[1]) {
+    const size_t bytes = shared_bytes(cap);
     k_ball_block<<<std::min(h[0], unsigned(ctx->sm_count) * 4u), BALL_BLOCK, bytes, s>>>(
         all, cent, rep, large.p, h[0], radius, sums, cap, mx.p + 1, mx.p + 2, ctx->d_status);
     CK(cudaGetLastError());
