@@ -36,18 +36,18 @@ __global__ void __launch_bounds__(128) k_bounded_all(const __grid_constant__ Mes
                                                      const __grid_constant__ Pose16 pose,
                                                      float window, double *out, uint32_t *status) {
   __shared__ unsigned next;
-  __shared__ WalkSlots<false> slots[4];
+  __shared__ WalkSlots slots[4];
   if (threadIdx.x == 0) next = 0;
   __syncthreads();
   uint32_t st = 0, first;
   const uint32_t count = block_share(n, first);
-  face_walks<false, false>(
+  face_walks(
       &next, count, slots[threadIdx.x >> 5],
       [&](uint32_t k, FaceWalk &w) {
         const size_t i = first + k;
         double x, y, z;
         apply_pose(pose.m, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], x, y, z);
-        return walk_start<false>(w, &m, {float(x), float(y), float(z)}, window);
+        return walk_start(w, &m, {float(x), float(y), float(z)}, window);
       },
       [&](uint32_t k, const FaceWalk &w) {
         out[size_t(first) + k] = w.best == f_inf() ? d_inf() : double(w.best);
@@ -361,7 +361,7 @@ __global__ void k_penetration_share(MeshView m, const double *pts, uint32_t n, P
       F3 p = {float(x), float(y), float(z)};
       bool in_box = !(p.x < m.lo[0] || p.x > m.hi[0] || p.y < m.lo[1] || p.y > m.hi[1] ||
                       p.z < m.lo[2] || p.z > m.hi[2]);
-      if (in_box && inside_mesh(m, p, st))
+      if (in_box && inside_mesh(m, p))
         deeper = double(mesh_distance(m, p, f_inf(), st)) > pen;
     }
     unsigned ballot = __ballot_sync(0xFFFFFFFFu, deeper);
@@ -892,7 +892,7 @@ __global__ void __launch_bounds__(INSIDE_BLOCK) k_inside(const __grid_constant__
   __shared__ unsigned next, found, parity[INSIDE_BLOCK / 32];
   __shared__ unsigned char queue[INSIDE_BLOCK];
   __shared__ float4 at[INSIDE_BLOCK];
-  __shared__ WalkSlots<false> slots[INSIDE_BLOCK / 32];
+  __shared__ WalkSlots slots[INSIDE_BLOCK / 32];
   const int warp = threadIdx.x >> 5;
   uint32_t st = 0;
   for (size_t first = size_t(blockIdx.x) * INSIDE_BLOCK; first < n;
@@ -917,11 +917,11 @@ __global__ void __launch_bounds__(INSIDE_BLOCK) k_inside(const __grid_constant__
       out[i] = {0.0f, 0u};
     }
     __syncthreads();
-    face_walks<false, false>(
+    face_walks(
         &next, found, slots[warp],
         [&](uint32_t k, FaceWalk &w) {
           const float4 q = at[queue[k]];
-          return walk_start<false>(w, &m, {q.x, q.y, q.z}, f_inf());
+          return walk_start(w, &m, {q.x, q.y, q.z}, f_inf());
         },
         [&](uint32_t k, const FaceWalk &w) { out[first + queue[k]] = {w.best, 1u}; }, st);
     __syncthreads();
@@ -945,8 +945,8 @@ __global__ void __launch_bounds__(256, PEN_INSIDE_MINB) k_pen_inside(const PairV
                                                     unsigned long long budget, uint32_t *status) {
   __shared__ WarpQueue wqs[8];
   __shared__ unsigned parity[8];
-  __shared__ WalkSlots<false> walk_slots[8];
-  WalkSlots<false> &slots = walk_slots[threadIdx.x >> 5];
+  __shared__ WalkSlots walk_slots[8];
+  WalkSlots &slots = walk_slots[threadIdx.x >> 5];
   WarpQueue &q = wqs[threadIdx.x >> 5];
   unsigned *par_word = parity + (threadIdx.x >> 5);
   int lane = threadIdx.x & 31;

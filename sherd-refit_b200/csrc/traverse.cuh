@@ -153,7 +153,7 @@ __device__ __noinline__ void first_hit(const MeshView &m, F3 o, F3 d, float &bes
 // such face was binned into p's cell of the axis grid (rectangle containment
 // implies cell containment, the cell index being monotone in the coordinate),
 // so scanning that one cell is the whole traversal.
-__device__ __noinline__ uint32_t crossings_axis(const MeshView &m, F3 p, int axis, uint32_t &status) {
+__device__ __noinline__ uint32_t crossings_axis(const MeshView &m, F3 p, int axis) {
   if (m.nf == 0) return 0;
   const AxisGrid &g = m.grid[axis];
   float pc[3] = {p.x, p.y, p.z};
@@ -172,18 +172,17 @@ __device__ __noinline__ uint32_t crossings_axis(const MeshView &m, F3 p, int axi
     tri_at(m, __ldg(g.slot + k), a, b1, c, id);
     if (moller_trumbore_edges(p, d, a, sub(b1, a), sub(c, a)) >= 0.0f) ++hits;
   }
-  (void)status;
   return hits;
 }
 
 // RayScene::inside (spatial/bvh.rs:146-157): the majority of three parities.
 // When the first two agree the third cannot change the majority, so it is
 // cast only when they differ.
-__device__ __forceinline__ bool inside_mesh(const MeshView &m, F3 p, uint32_t &status) {
-  uint32_t a = crossings_axis(m, p, 0, status) & 1u;
-  uint32_t b = crossings_axis(m, p, 1, status) & 1u;
+__device__ __forceinline__ bool inside_mesh(const MeshView &m, F3 p) {
+  uint32_t a = crossings_axis(m, p, 0) & 1u;
+  uint32_t b = crossings_axis(m, p, 1) & 1u;
   if (a == b) return a != 0;
-  return (crossings_axis(m, p, 2, status) & 1u) != 0;
+  return (crossings_axis(m, p, 2) & 1u) != 0;
 }
 
 __device__ __forceinline__ float box_dist2(const float *lo, const float *hi, const float *p) {
@@ -432,28 +431,12 @@ __device__ __noinline__ float mesh_nearest_face(const MeshView &m, F3 p, float w
 // PointTree::nearest_within_squared (spatial/kdtree.rs:202-217): the nearest
 // point with d2 <= r2, lowest original index on an exact tie. Returns the
 // sorted slot (or -1) and its squared distance; d2 = ((dx dx + dy dy) + dz dz).
-//
-// `hint` (a sorted slot, or -1) seeds the search with a point that is already
-// a candidate, typically the previous ICP pass's match: its exact distance is
-// the initial bound, so the traversal prunes from the first node. The answer
-// is the same with or without it: the hint is a valid candidate, anything
-// nearer replaces it, and an exact tie still goes to the lower index.
 __device__ __noinline__ int nearest_within_sq(const CloudView &c, double qx, double qy, double qz, double r2,
-                                 double &best, uint32_t &status, int hint = -1) {
+                                 double &best, uint32_t &status) {
   best = r2;
   int best_s = -1;
   uint32_t best_i = MISS;
   if (c.n == 0 || !(r2 >= 0.0)) return -1;
-  if (hint >= 0) {
-    double4 p = ldg4(c.pts + hint);
-    double dx = qx - p.x, dy = qy - p.y, dz = qz - p.z;
-    double d2 = (dx * dx + dy * dy) + dz * dz;
-    if (d2 <= r2) {
-      best = d2;
-      best_s = hint;
-      best_i = uint32_t(p.w);
-    }
-  }
   float qc[3] = {float(qx), float(qy), float(qz)};
   auto bound2 = [&]() {
     float b = __double2float_ru(best);

@@ -78,7 +78,7 @@ struct VerShared {
   unsigned best_key;
   unsigned deep_key;
   unsigned next;  // the next query of one_side
-  WalkSlots<false> walk[32];
+  WalkSlots walk[32];
   unsigned cells[MAX_CELL_WORDS];
 };
 
@@ -201,13 +201,13 @@ __device__ __noinline__ void one_side(const double4 *pts, uint32_t n, const doub
   __syncthreads();
   const float window = float(sc.facing);
   unsigned tight_n = 0, touching = 0;
-  face_walks<false, false>(
+  face_walks(
       &sh.next, n, sh.walk[threadIdx.x >> 5],
       [&](uint32_t i, FaceWalk &w) {
         double4 q = ldg4(pts + i);
         double x, y, z;
         apply_pose(pose, q.x, q.y, q.z, x, y, z);
-        return walk_start<false>(w, &scene, narrow3(x, y, z), window);
+        return walk_start(w, &scene, narrow3(x, y, z), window);
       },
       [&](uint32_t, const FaceWalk &w) {
         const float d = w.best;
@@ -463,7 +463,7 @@ __device__ __noinline__ void one_penetration(const double4 *pts, uint32_t n, con
     unsigned nb = sh.n_box;
     for (uint32_t k = threadIdx.x; k < nb; k += blockDim.x) {
       uint32_t i = sh.q_box[k];
-      warp_append(inside_mesh(scene, moved_point(pts, i, pose), status), i, sh.q_in, &sh.n_in);
+      warp_append(inside_mesh(scene, moved_point(pts, i, pose)), i, sh.q_in, &sh.n_in);
     }
     __syncthreads();
     unsigned ni = sh.n_in;

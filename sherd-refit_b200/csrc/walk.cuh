@@ -7,9 +7,8 @@
 // query (when WALK_REFILL of them are idle), and the faces of the leaves the
 // lanes have come to are laid end to end and tested by all of them.
 //
-// The answers are mesh_distance's and mesh_nearest_face's: every face within the
-// padded bound is tested, whatever the order, and the smallest distance (the
-// lowest face id on a tie) within the window is kept.
+// The answers are mesh_distance's: every face within the padded bound is tested,
+// whatever the order, and the smallest distance within the window is kept.
 #pragma once
 
 #include "traverse.cuh"
@@ -24,7 +23,6 @@ struct FaceWalk {
   float window;    // distances above it do not count
   float best;      // the smallest so far within it, +inf before
   float bound2;    // the padded square of the bound boxes are held against
-  uint32_t id, slot;  // its face (NEAREST only)
   int node, sp;
   uint32_t visits;
 };
@@ -41,13 +39,12 @@ __device__ __forceinline__ void walk_bound(FaceWalk &w) {
 
 // Starts the query of p against m within the window; false when it is answered
 // already (w.best): nothing to find, or a mesh of one leaf.
-template <bool NEAREST, bool ANY = false>
+template <bool ANY = false>
 __device__ __forceinline__ bool walk_start(FaceWalk &w, const MeshView *m, F3 p, float window) {
   w.m = m;
   w.p = p;
   w.window = window;
   w.best = f_inf();
-  w.id = w.slot = MISS;
   w.node = w.sp = 0;
   w.visits = 0;
   if (m->nf == 0 || !(ANY ? window >= 0.0f : window > 0.0f)) return false;
@@ -61,31 +58,20 @@ __device__ __forceinline__ bool walk_start(FaceWalk &w, const MeshView *m, F3 p,
     uint32_t id;
     tri_at(*m, s, a, b, c, id);
     const float d = tri_distance(p, a, b, c);
-    if (d <= window && (d < w.best || (NEAREST && d == w.best && id < w.id))) {
-      w.best = d;
-      w.id = id;
-      w.slot = s;
-    }
+    if (d <= window && d < w.best) w.best = d;
   }
   return false;
 }
 
 // A warp's shared words for its leaves.
-template <bool NEAREST>
 struct WalkSlots {
   unsigned key[32];
-};
-template <>
-struct WalkSlots<true> {
-  unsigned long long key[32];
-  uint32_t slot[32];
 };
 
 // The faces [first, first + count) of each lane's leaf (count 0: none) tested
 // against its point by all lanes, and its walk's best brought up to date.
-template <bool NEAREST>
 __device__ __forceinline__ void walk_leaves(FaceWalk &w, uint32_t first, uint32_t count,
-                                            WalkSlots<NEAREST> &sh) {
+                                            WalkSlots &sh) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   uint32_t incl = count;
@@ -95,10 +81,7 @@ __device__ __forceinline__ void walk_leaves(FaceWalk &w, uint32_t first, uint32_
     if (lane >= o) incl += y;
   }
   const uint32_t off = incl - count, total = __shfl_sync(FULL, incl, 31);
-  if constexpr (NEAREST)
-    sh.key[lane] = (unsigned long long)f2key(w.best) << 32 | w.id;
-  else
-    sh.key[lane] = f2key(w.best);
+  sh.key[lane] = f2key(w.best);
   __syncwarp();
   const unsigned long long tri = reinterpret_cast<unsigned long long>(count ? w.m->tri : nullptr);
   for (uint32_t base = 0; base < total; base += 32) {
@@ -110,50 +93,26 @@ __device__ __forceinline__ void walk_leaves(FaceWalk &w, uint32_t first, uint32_
     const F3 q = {__shfl_sync(FULL, w.p.x, j), __shfl_sync(FULL, w.p.y, j), __shfl_sync(FULL, w.p.z, j)};
     const float window = __shfl_sync(FULL, w.window, j);
     const uint32_t fj = __shfl_sync(FULL, first, j), oj = __shfl_sync(FULL, off, j);
-    const uint32_t s = fj + (e - oj);
-    const float4 *t = reinterpret_cast<const float4 *>(__shfl_sync(FULL, tri, j)) + 3 * size_t(s);
-    unsigned long long mine = ~0ull;
+    const float4 *t = reinterpret_cast<const float4 *>(__shfl_sync(FULL, tri, j)) + 3 * size_t(fj + (e - oj));
     if (e < total) {
       const float4 a = __ldg(t), b = __ldg(t + 1), c = __ldg(t + 2);
       const float d = tri_distance(q, {a.x, a.y, a.z}, {b.x, b.y, b.z}, {c.x, c.y, c.z});
-      if (d <= window) {
-        if constexpr (NEAREST) {
-          mine = (unsigned long long)f2key(d) << 32 | __float_as_uint(a.w);
-          atomicMin(&sh.key[j], mine);
-        } else {
-          atomicMin(&sh.key[j], f2key(d));
-        }
-      }
-    }
-    if constexpr (NEAREST) {
-      __syncwarp();
-      if (e < total && mine != ~0ull && sh.key[j] == mine) sh.slot[j] = s;
-      __syncwarp();
+      if (d <= window) atomicMin(&sh.key[j], f2key(d));
     }
   }
   __syncwarp();
-  if (count) {
-    if constexpr (NEAREST) {
-      const unsigned long long k = sh.key[lane];
-      if (k != ((unsigned long long)f2key(w.best) << 32 | w.id)) {
-        w.best = key2f(unsigned(k >> 32));
-        w.id = uint32_t(k);
-        w.slot = sh.slot[lane];
-        walk_bound(w);
-      }
-    } else if (key2f(sh.key[lane]) < w.best) {
-      w.best = key2f(sh.key[lane]);
-      walk_bound(w);
-    }
+  if (count && key2f(sh.key[lane]) < w.best) {
+    w.best = key2f(sh.key[lane]);
+    walk_bound(w);
   }
   __syncwarp();
 }
 
 // One node of every lane's walk (`active`: it has one); false where it has ended.
 // ANY: a walk ends with the first face it finds.
-template <bool NEAREST, bool ANY>
+template <bool ANY>
 __device__ __forceinline__ bool walk_step(FaceWalk &w, bool active, int *stack_n, float *stack_k,
-                                          WalkSlots<NEAREST> &sh, uint32_t &st) {
+                                          WalkSlots &sh, uint32_t &st) {
   if (active && ++w.visits > 2u * w.m->nf + 64u) {
     st |= ST_STACK;
     active = false;
@@ -184,7 +143,7 @@ __device__ __forceinline__ bool walk_step(FaceWalk &w, bool active, int *stack_n
       next = go0 ? n.ref[0] : n.ref[1];
     }
   }
-  if (__any_sync(0xffffffffu, faces != 0)) walk_leaves<NEAREST>(w, first, faces, sh);
+  if (__any_sync(0xffffffffu, faces != 0)) walk_leaves(w, first, faces, sh);
   if (!active || (ANY && w.best != f_inf())) return false;
   if (next < 0) {
     while (w.sp > 0) {
@@ -201,9 +160,9 @@ __device__ __forceinline__ bool walk_step(FaceWalk &w, bool active, int *stack_n
 
 // The queries [0, n) of a block (or of one warp), handed out from *counter:
 // `start(i, w)` starts query i and says whether it has to walk, `done(i, w)`
-// takes its answer (w.best, w.slot). Every lane of the warp calls it.
-template <bool NEAREST, bool ANY, class Start, class Done>
-__device__ __forceinline__ void face_walks(unsigned *counter, uint32_t n, WalkSlots<NEAREST> &sh,
+// takes its answer (w.best). Every lane of the warp calls it.
+template <class Start, class Done>
+__device__ __forceinline__ void face_walks(unsigned *counter, uint32_t n, WalkSlots &sh,
                                            Start &&start, Done &&done, uint32_t &st) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -230,7 +189,7 @@ __device__ __forceinline__ void face_walks(unsigned *counter, uint32_t n, WalkSl
     }
     if (idle == FULL) return;
     const bool was = active;
-    active = walk_step<NEAREST, ANY>(w, active, stack_n, stack_k, sh, st);
+    active = walk_step<false>(w, active, stack_n, stack_k, sh, st);
     if (was && !active) done(i, w);
   }
 }
@@ -244,14 +203,14 @@ __device__ __forceinline__ void face_walks(unsigned *counter, uint32_t n, WalkSl
 // is none.
 template <bool ANY>
 __device__ __noinline__ float warp_walks(const MeshView *m, F3 p, float window, bool need,
-                                         WalkSlots<false> &sh, uint32_t &st) {
+                                         WalkSlots &sh, uint32_t &st) {
   int stack_n[STACK];
   float stack_k[STACK];
   FaceWalk w;
   w.best = f_inf();
-  bool active = need && walk_start<false, ANY>(w, m, p, window);
+  bool active = need && walk_start<ANY>(w, m, p, window);
   while (__any_sync(0xffffffffu, active))
-    active = walk_step<false, ANY>(w, active, stack_n, stack_k, sh, st);
+    active = walk_step<ANY>(w, active, stack_n, stack_k, sh, st);
   return w.best;
 }
 
