@@ -46,8 +46,8 @@ L2_FLUSH_BYTES = 256 << 20
 # it was taken on: a capture of other sources is not reported.
 TRAFFIC = {
     # the ladder stage's bucket launches together (> 16384 and > 4096 moving points; ncu runs
-    # them one after the other): 104.48 + 147.47 GB read, 26.85 + 123.78 GB written
-    ("collection", 0, "k_ladder", 1): (402.58e9, "bbb2f9119671"),
+    # them one after the other): 18.19 + 43.06 GB read, 12.70 + 61.34 GB written
+    ("collection", 0, "k_ladder", 1): (135.29e9, "4eb5b149f49b"),
 }
 
 
@@ -138,7 +138,8 @@ def nn_query_rates(sbytes: dict, stage_ms: dict, step_ms: float, total_q: float)
             "nn_queries_per_s": q / (ms / 1000.0) if ms > 0 else None,
             "nn_queries_per_s_whole_step": total_q / (step_ms / 1000.0) if step_ms > 0 else None,
             "unit": "queries/s",
-            "what": "one bounded nearest-neighbour query per ICP point-iteration (k_ladder)"}
+            "what": ("one bounded nearest-neighbour query per ICP point-iteration (k_ladder), answered "
+                     "by a search or by proof that the last match still stands")}
 
 
 CPU_ITEMS = 512
@@ -784,7 +785,12 @@ def main():
     rec = TRAFFIC.get((args.config, args.seed, kernel_of[dom], world))
     traffic = rec[0] if rec and rec[1] == src else None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak, "traffic": traffic,
+                "frac": achieved / peak,
+                "of": ("algorithmic bytes: a count of the work asked for, whether or not a kept "
+                       "match let a chunk of points go unread; not a measure of traffic"),
+                "traffic": traffic,
+                "traffic_gbs": (traffic / (stages[dom]["ms"] / 1000.0) / 1e9
+                                if traffic and stages[dom]["ms"] > 0 else None),
                 "traffic_source": (f"ncu dram__bytes_read.sum + dram__bytes_write.sum of the "
                                    f"stage's launches in one full-size step of this build (CUDA "
                                    f"sources {src})"

@@ -505,9 +505,7 @@ __device__ __forceinline__ int hint_load(const H *h, uint32_t i) {
 // nearest_within_sq that also says how far the point may move before its
 // match can change: `slack` receives a lower bound on the distance from the
 // query to every target point but the match (to every point when there is
-// none): the nearest of what was scored and of what was left out, and the
-// search reaches `margin` past the best so far, so what is left out is at least
-// that far.
+// none): the nearest of what was scored and of the boxes that were left out.
 // (Box distances come from the f32-rounded query; the boxes' padding, or far
 // from the cloud the 1e-5, covers that.)
 __device__ __noinline__ int nearest_guarded(const CloudView &c, double qx, double qy, double qz,

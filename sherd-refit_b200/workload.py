@@ -104,7 +104,9 @@ def pair_n_src(wl) -> np.ndarray:
 
 def stage_bytes(wl, cands, n_src=None):
     """Compulsory bytes of each stage of the batched path over the units in `cands` (their pair
-    field indexing wl.pairs, and n_src by default that of every workload pair):
+    field indexing wl.pairs, and n_src by default that of every workload pair). A count of the
+    work asked for, not of memory traffic: a rung's pass leaves chunks unread whose points
+    provably match nothing, and the trees' own reads are not in it.
     ladder: 48 B per ICP point-iteration (16 B source point, 32 B matched target point and
     normal) over the passes each rung ran (iterations + 1); verify: 24 B per query of
     |Pf_A| + |Pf_B| + |brk_A| + |Pm_B|; pen_inside: 24 B per surface sample |S_A| + |S_B|;
