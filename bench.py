@@ -127,6 +127,15 @@ def _max_over_ranks(world, x):
     return x if world == 1 else _pkg("shard").max_over_ranks(x, device="cuda")
 
 
+def stage_launches(n_src, n_items: int) -> int:
+    """Kernel launches of one step of the batched schedule over pairs of n_src (n, 2) moving
+    points: a k_ladder per point-count bucket (> 16384, > 4096, the rest) that has items, one
+    launch or two of the verification, five of the penetration."""
+    most = np.asarray(n_src).max(axis=1)
+    buckets = len(np.unique((most > 16384) * 2 + ((most > 4096) & (most <= 16384))))
+    return buckets + (1 if n_items > 74 else 2) + 5
+
+
 def nn_query_rates(sbytes: dict, stage_ms: dict, step_ms: float, total_q: float) -> dict:
     """NN queries/s of the batched path: every ICP point-iteration of k_ladder is one bounded
     nearest-neighbour query (48 algorithmic bytes each), so the ladder stage's queries are its
@@ -832,9 +841,11 @@ def main():
                           "and candidates into pinned host buffers allocated once) and the "
                           "candidate all-gather (max over ranks); bytes per rank"),
                 "matches_resident_run": same},
-        "gpu_launches": 9 * args.steps,
-        "gpu_launches_counts": ("per step: k_ladder once per point-count bucket (3), "
-                                "k_verify_items, k_pen_init, k_pen_inside, k_pen_seed, k_pen_min, "
+        "gpu_launches": stage_launches(workload.pair_n_src(wl)[np.asarray(dev.pair_index)],
+                                       dev.n_items) * args.steps,
+        "gpu_launches_counts": ("per step: k_ladder once per point-count bucket that has items, "
+                                "k_verify_items (k_verify_parts and k_verify_join for 74 items or "
+                                "fewer), k_pen_init, k_pen_inside, k_pen_seed, k_pen_min, "
                                 "k_pen_finalize"),
         "ladder_autotune": ctx.stats().get("ladder_autotune"),
         "nn_queries": nn_query_rates(sbytes, stage_ms, step_ms, total_q),

@@ -57,3 +57,14 @@ def test_both_arms_describe_the_workload_alike(monkeypatch):
     a = bench._config_dict(wl, Args())
     b = bench._config_dict(wl, Args())
     assert a == b and a["items"] == 16 and "strong scaling" in a["parallelism"]
+
+
+def test_launches_are_counted_by_the_buckets_that_have_items():
+    """A ladder launch per point-count bucket in use, a verification in one launch or, for few
+    items, in two, and five penetration kernels."""
+    bench = _bench()
+    mid, large, small = [6000, 5000], [100, 16385], [4096, 7]
+    assert bench.stage_launches([mid, large, mid], 99840) == 8
+    assert bench.stage_launches([mid], 1792) == 7
+    assert bench.stage_launches([small, mid, large], 75) == 9
+    assert bench.stage_launches([[16384, 4097]], 74) == 8
