@@ -437,6 +437,17 @@ int mesh_build(sherd_ctx *ctx, sherd_mesh *m) {
   if (rc) return rc;
   rc = upload(ctx, df, m->hf.data(), m->hf.size());
   if (rc) return rc;
+  // The edges are summed up on the device: the host's loop over them was 3 of the 13 ms
+  // that a mesh of 998,000 faces took to build.
+  const unsigned edge_blocks = std::min(blocks_for(nf, EDGE_BLOCK), EDGE_BLOCKS);
+  std::vector<double2> edge_part(edge_blocks);
+  DBuf<double2> dpart;
+  CK(dpart.alloc(edge_blocks));
+  k_edge_sums<<<edge_blocks, EDGE_BLOCK, 0, ctx->stream>>>(dv.p, df.p, nf, dpart.p);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(edge_part.data(), dpart.p, sizeof(double2) * edge_blocks, cudaMemcpyDeviceToHost,
+                     ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
   double mag = 1.0;
   for (float x : m->hv) mag = std::max(mag, double(std::fabs(x)));
   float pad = float(1e-5 * mag);
@@ -457,33 +468,29 @@ int mesh_build(sherd_ctx *ctx, sherd_mesh *m) {
   // are a quarter of the mean edge across: of the entries of cells a mean edge
   // across nine in ten missed the point. (Cells of 1 / 0.5 / 0.35 / 0.25 edges: the
   // inside pass of 28,224 items 90 / 77 / 76 / 72 ms, of 1,792 items 20.3 / 17.6 /
-  // 16.5 / 16.0, 20,000 inside queries 321 / 236 / 225 / 200 us; the build of a
-  // mesh within 2 %.) A face's entries grow as the square of its size in cells, so
+  // 16.5 / 16.0, 20,000 inside queries 321 / 236 / 225 / 200 us; the build of a mesh
+  // of 16,000, 129,000 and 998,000 faces 0.73, 1.98 and 9.1 ms, 0.76, 1.96 and 9.1 with
+  // cells of the mean edge.) A face's entries grow as the square of its size in cells, so
   // a mesh with faces far larger than its mean edge, or within its padding, gets
   // coarser cells, down to the mean edge: the mean square of two edges and the
   // padding's width, which is a quarter of a face's rectangle or more, stays
   // below GRID_SQUARES cells.
   double edge = 0.0, squares = 0.0;
-  auto square = [](const float *a, const float *b) {
-    const double x = a[0] - b[0], y = a[1] - b[1], z = a[2] - b[2];
-    return x * x + y * y + z * z;
-  };
-  for (uint32_t i = 0; i < nf; ++i) {
-    const float *b = &m->hv[3 * m->hf[3 * i + 1]];
-    const double ab = square(&m->hv[3 * m->hf[3 * i]], b);
-    edge += std::sqrt(ab);
-    squares += ab + square(b, &m->hv[3 * m->hf[3 * i + 2]]);
+  for (const double2 &p : edge_part) {
+    edge += p.x;
+    squares += p.y;
   }
   const double faces = std::max<uint32_t>(nf, 1);
   edge = std::max(edge / faces, 1e-6);
   squares = squares / (2.0 * faces) + 4.0 * double(pad) * pad;
-  AxisGrid grids[3] = {};
+  GridBuild build = {};
+  const dim3 face_blocks(blocks_for(nf), 3);
   DBuf<unsigned> count[3], dtotal;
   uint32_t total[3] = {};
   CK(dtotal.alloc(3));
   for (int axis = 0; axis < 3; ++axis) {
     int au = (axis + 1) % 3, av = (axis + 2) % 3;
-    AxisGrid &g = grids[axis];
+    AxisGrid &g = build.grid[axis];
     double lo_u = double(vlo[au]) - 2.0 * pad, lo_v = double(vlo[av]) - 2.0 * pad;
     double ext_u = double(vhi[au]) - lo_u + 2.0 * pad, ext_v = double(vhi[av]) - lo_v + 2.0 * pad;
     double cell = edge / 4.0;
@@ -498,8 +505,12 @@ int mesh_build(sherd_ctx *ctx, sherd_mesh *m) {
     size_t cells = size_t(g.nu) * g.nv;
     CK(count[axis].alloc(cells + 1));
     CK(cudaMemsetAsync(count[axis].p, 0, sizeof(unsigned) * (cells + 1), ctx->stream));
-    k_grid_count<<<blocks_for(nf), 256, 0, ctx->stream>>>(m->tri.p, nf, axis, g, pad, count[axis].p);
-    CK(cudaGetLastError());
+    build.count[axis] = count[axis].p;
+  }
+  k_grid_count<<<face_blocks, 256, 0, ctx->stream>>>(m->tri.p, nf, build, pad);
+  CK(cudaGetLastError());
+  for (int axis = 0; axis < 3; ++axis) {
+    const size_t cells = count[axis].n - 1;
     CK(m->gstart[axis].alloc(cells + 1));
     size_t temp_bytes = 0;
     CK(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, count[axis].p, m->gstart[axis].p, int(cells + 1),
@@ -511,24 +522,25 @@ int mesh_build(sherd_ctx *ctx, sherd_mesh *m) {
     CK(cudaMemcpyAsync(dtotal.p + axis, m->gstart[axis].p + cells, 4, cudaMemcpyDeviceToDevice,
                        ctx->stream));
   }
-  // The entries' numbers, to size them: the one wait of a build.
+  // The entries' numbers, to size them.
   CK(cudaMemcpyAsync(total, dtotal.p, sizeof total, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   for (int axis = 0; axis < 3; ++axis) {
-    AxisGrid &g = grids[axis];
+    AxisGrid &g = build.grid[axis];
     const size_t entries = std::max<uint32_t>(total[axis], 1);
     CK(m->grect[axis].alloc(entries));
     CK(m->gslot[axis].alloc(entries));
     CK(cudaMemcpyAsync(count[axis].p, m->gstart[axis].p, sizeof(unsigned) * size_t(g.nu) * g.nv,
                        cudaMemcpyDeviceToDevice, ctx->stream));
-    k_grid_fill<<<blocks_for(nf), 256, 0, ctx->stream>>>(m->tri.p, nf, axis, g, pad, count[axis].p,
-                                                        m->grect[axis].p, m->gslot[axis].p);
-    CK(cudaGetLastError());
+    build.rect[axis] = m->grect[axis].p;
+    build.slot[axis] = m->gslot[axis].p;
     g.start = m->gstart[axis].p;
     g.rect = m->grect[axis].p;
     g.slot = m->gslot[axis].p;
     m->view.grid[axis] = g;
   }
+  k_grid_fill<<<face_blocks, 256, 0, ctx->stream>>>(m->tri.p, nf, build, pad);
+  CK(cudaGetLastError());
   MeshView &v = m->view;
   v.nodes = m->nodes.p;
   v.tri = m->tri.p;

@@ -73,3 +73,39 @@ def test_queries_are_bit_exact(gpu_ctx, oracle, name, n):
     for window in (0.0, float(0.05 * half.min()), float(half.max()), np.inf):
         assert np.array_equal(gpu_ctx.bounded_distance(g, pts, pose, window),
                               c.bounded_distance(pts, pose, window)), window
+
+
+def _soup(n, large):
+    """n loose faces, `large` of them of about sixty times the others' size."""
+    rng = np.random.default_rng(n)
+    size = np.where(np.arange(n) < large, 3.0, 0.05)[:, None, None]
+    v = rng.uniform(-10, 10, size=(n, 1, 3)) + rng.normal(size=(n, 3, 3)) * size
+    return v.reshape(-1, 3), np.arange(3 * n).reshape(-1, 3)
+
+
+@pytest.mark.parametrize("n,large", [(1, 1), (31, 3), (33, 32), (257, 5), (3001, 30)])
+def test_parities_among_faces_of_any_size(gpu_ctx, oracle, n, large):
+    """Faces of one cell and of thousands side by side in a warp of the grids' build."""
+    v, f = _soup(n, large)
+    q = np.random.default_rng(n + 1).uniform(-12, 12, size=(5000, 3))
+    gd, gi = gpu_ctx.inside(gpu_ctx.mesh(v, f), q, np.eye(4))
+    cd, ci = oracle.Mesh(v, f).inside(q, np.eye(4))
+    assert np.array_equal(gi, ci)
+    assert np.array_equal(np.asarray(gd).view(np.uint32), np.asarray(cd).view(np.uint32))
+
+
+def test_a_few_large_faces_do_not_hold_up_a_mesh(gpu_ctx):
+    """A mesh with one large face in a hundred is built in the time of one without, and not in
+    that of a thread that goes through the largest face's cells (seven times as long)."""
+    import time
+
+    def build(v, f):
+        best = np.inf
+        for _ in range(8):
+            t0 = time.perf_counter()
+            mesh = gpu_ctx.mesh(v, f)
+            best = min(best, time.perf_counter() - t0)
+            del mesh
+        return best
+    v, f = _soup(20000, 0)
+    assert build(*_soup(20000, 200)) < 3.0 * build(v, f)
