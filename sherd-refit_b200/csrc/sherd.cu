@@ -1597,6 +1597,7 @@ int sherd_pair_free(sherd_pair *pair) {
 struct sherd_batch {
   sherd_ctx *ctx = nullptr;
   bool verify_only = false;  // no ladder, and nothing stops it
+  bool pen = true;           // the penetration is asked for
   StopCtl stop() const { return verify_only ? StopCtl{} : ctx->stop_ctl(); }
   unsigned long long budget() const {
     return verify_only ? 0ull : (unsigned long long)ctx->timeout_ms * 1000000ULL;
@@ -1972,7 +1973,9 @@ int batch_create(sherd_ctx *ctx, const std::vector<PairView> &views, const sherd
   CK(b->heads.alloc(sherd_batch::HEADS * size_t(std::max<uint32_t>(n_pairs, 1))));
   int occ_v = 0;
   const int threads = 2 * ICP_BLOCK;
-  if (b->hint16) {
+  if (b->verify_only) {
+    // no ladder to size
+  } else if (b->hint16) {
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[0], k_ladder<uint16_t, 2, 1, LADDER_MINB[0]>, threads, 0));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[1], k_ladder<uint16_t, 2, 1, LADDER_MINB[1]>, threads, 0));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ[2], k_ladder<uint16_t, 2, 1, LADDER_MINB[2]>, threads, 0));
@@ -1991,7 +1994,8 @@ int batch_create(sherd_ctx *ctx, const std::vector<PairView> &views, const sherd
   uint32_t blocks_v = std::min(most, b->grid_v);
   if (sched == SHERD_SCHED_BATCHED && !b->early() && verify_in_parts(b, n_items)) blocks_v = 4 * n_items;
   CK(b->scratch.alloc(size_t(std::max(1u, blocks_v)) * b->max_scratch));
-  if (sched == SHERD_SCHED_BATCHED) {
+  if (sched == SHERD_SCHED_BATCHED) CK(b->inv.alloc(16 * size_t(n_items)));
+  if (sched == SHERD_SCHED_BATCHED && b->pen) {
     // Unit 2i is item i's side 0 (B's samples in A's mesh), 2i+1 its side 1.
     std::vector<uint32_t> chunk0(2 * size_t(n_items) + 1);
     uint64_t acc = 0;
@@ -2017,7 +2021,6 @@ int batch_create(sherd_ctx *ctx, const std::vector<PairView> &views, const sherd
       coarse[k] = cu;
     }
     if ((rc = upload(ctx, b->coarse, coarse.data(), coarse.size()))) return rc;
-    CK(b->inv.alloc(16 * size_t(n_items)));
     CK(b->deeper.alloc(2 * size_t(n_items)));
     CK(b->deep.alloc(2 * size_t(n_items)));
     CK(b->best.alloc(2 * size_t(n_items)));
@@ -2028,6 +2031,7 @@ int batch_create(sherd_ctx *ctx, const std::vector<PairView> &views, const sherd
     b->grid_p = unsigned(std::max(1, occ_p) * ctx->sm_count);
     b->grid_m = unsigned(std::max(1, occ_m) * ctx->sm_count);
   }
+  if (b->verify_only) return SHERD_OK;
   b->hint_stride = (b->hint_stride + 63) / 64 * 64;
   // A slot for every item in flight: the plain schedule launches one block or
   // cluster per item of a pair, early rejection up to grid_l of them.
@@ -2054,7 +2058,7 @@ int batch_create(sherd_ctx *ctx, const std::vector<PairView> &views, const sherd
   CK(b->mem.alloc(b->hint_stride, slots, ints ? sizeof(int) : sizeof(uint16_t)));
   for (cudaEvent_t &e : b->ev) CK(cudaEventCreate(&e));
   CK(cudaStreamSynchronize(ctx->stream));
-  if (sched == SHERD_SCHED_BATCHED && !b->verify_only) {
+  if (sched == SHERD_SCHED_BATCHED) {
     if (!b->early() && (rc = tune_ladder(b))) return rc;
     if (resident) return capture(b);
   }
@@ -2161,6 +2165,7 @@ int sherd_verify(sherd_ctx *ctx, const sherd_surfaces *a, const sherd_surfaces *
   p.early_reject_tight = 0.0;
   sherd_batch one;
   one.verify_only = true;
+  one.pen = full != 0;
   if ((rc = batch_create(ctx, views, &item, 1, &p, SHERD_SCHED_BATCHED, false, &one))) return rc;
   CK(cudaMemcpyAsync(one.dc.p, &cand, sizeof cand, cudaMemcpyHostToDevice, ctx->stream));
   if ((rc = launch_verify(&one, ctx->stream, full ? 1 : 0))) return rc;
