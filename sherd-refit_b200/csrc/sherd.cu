@@ -445,12 +445,12 @@ int mesh_build(sherd_ctx *ctx, sherd_mesh *m) {
   CK(dpart.alloc(edge_blocks));
   k_edge_sums<<<edge_blocks, EDGE_BLOCK, 0, ctx->stream>>>(dv.p, df.p, nf, dpart.p);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(edge_part.data(), dpart.p, sizeof(double2) * edge_blocks, cudaMemcpyDeviceToHost,
-                     ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
   double mag = 1.0;
   for (float x : m->hv) mag = std::max(mag, double(std::fabs(x)));
   float pad = float(1e-5 * mag);
+  CK(cudaMemcpyAsync(edge_part.data(), dpart.p, sizeof(double2) * edge_blocks, cudaMemcpyDeviceToHost,
+                     ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
   rc = build_lbvh<true>(ctx, dv.p, nv, df.p, nullptr, nf, pad, TRI_LEAF, m->nodes, sorted);
   if (rc) return rc;
   CK(m->tri.alloc(size_t(3) * nf));
