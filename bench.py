@@ -46,8 +46,8 @@ L2_FLUSH_BYTES = 256 << 20
 # it was taken on: a capture of other sources is not reported.
 TRAFFIC = {
     # the ladder stage's bucket launches together (> 16384 and > 4096 moving points; ncu runs
-    # them one after the other): 18.19 + 43.06 GB read, 12.70 + 61.34 GB written
-    ("collection", 0, "k_ladder", 1): (135.29e9, "4eb5b149f49b"),
+    # them one after the other): 18.11 + 43.66 GB read, 12.67 + 62.03 GB written
+    ("collection", 0, "k_ladder", 1): (136.47e9, "1e93542e4f92"),
 }
 
 
