@@ -125,12 +125,11 @@ def test_ladders_run_alike_in_every_form(sherd, gpu_ctx, gpu_slab, slab, n, limi
     """The queue's items shared by a cluster's blocks, in one launch or split by the early
     rejection: the same candidates on clusters of 8, 4 and 2 blocks, on wide blocks and on narrow
     ones, under both schedules."""
-    rng = np.random.default_rng(n)
-    tp, tn = _surface(rng, 3000)
-    src, _ = _surface(rng, n)
-    pair = gpu_ctx.pair(gpu_slab["a"]["surf"], gpu_slab["b"]["surf"], gpu_ctx.cloud(tp, tn),
-                        gpu_slab["frac_t"], src, src[:n // 2], gpu_slab["scales"])
-    inits = np.concatenate([slab["starts"].reshape(-1, 4, 4), _starts(rng, 20)])
+    b = gpu_slab["b"]["arrays"]  # its clouds, cut or repeated to n and n / 2 points
+    pair = gpu_ctx.pair(gpu_slab["a"]["surf"], gpu_slab["b"]["surf"], gpu_slab["reg_t"],
+                        gpu_slab["frac_t"], np.resize(b["reg_p"], (n, 3)),
+                        np.resize(b["frac_p"], (n // 2, 3)), gpu_slab["scales"])
+    inits = slab["starts"].reshape(-1, 4, 4)
     params = sherd.default_params()
     params.early_reject_tight = limit
 
@@ -138,6 +137,8 @@ def test_ladders_run_alike_in_every_form(sherd, gpu_ctx, gpu_slab, slab, n, limi
         items = [(0, i, inits[i % len(inits)]) for i in range(k)]
         return sherd.candidates(gpu_ctx.ladder_verify_batch([pair], items, params, sched)).copy()
     whole = run(max(STARTS), sherd.SCHED_BATCHED)
+    partial = int(whole["scores"]["partial"].sum())
+    assert 0 < partial < len(whole) if limit else partial == 0
     for k in STARTS * 2:
         for sched in (sherd.SCHED_BATCHED, sherd.SCHED_PLAIN):
             assert run(k, sched).tobytes() == whole[:k].tobytes(), (k, sched)
